@@ -102,7 +102,8 @@ typedef struct dem_ext {
                                          graphs with conditional nodes, and for hosts that capture the
                                          calls into graphs of their own); results do not depend on it */
     int32_t split_narrow;             /* 1: narrow phase and forces as two kernels (fewer registers
-                                         each; faster in dense scenes); results do not depend on it */
+                                         each); 0: the library's choice (two in dense contexts and
+                                         batches with bonds); results do not depend on it */
     int32_t unfused_lom;              /* 1: every step runs its own LOM kernel instead of the next
                                          step's LOM pass running inside the Simulation kernel (the
                                          default, fewer bytes per step); results do not depend on it */

@@ -82,6 +82,22 @@ __device__ __forceinline__ bool shared_bucket(const DevWorld &w, uint32_t ca, ui
     return true;
 }
 
+// a range with which shared_bucket may report device error 2 (a narrower one
+// keeps every rank below 16; a partner's own pass reports the partner's)
+__device__ __forceinline__ bool wide_range(uint32_t ca) {
+    const int wa = (int)((ca >> 22) & 31u), ha = (int)(ca >> 27);
+    return wa * ha > 16 || wa == 31 || ha == 31;
+}
+
+// shared_bucket without the rank and the error
+__device__ __forceinline__ bool shares_bucket(uint32_t ca, uint32_t cb) {
+    const int wa = (int)((ca >> 22) & 31u), ha = (int)(ca >> 27);
+    const int wb = (int)((cb >> 22) & 31u), hb = (int)(cb >> 27);
+    const int dx = (int)((cb - ca) << 21) >> 21;                  // bx0 - ax0
+    const int dy = (int)(((cb >> 11) - (ca >> 11)) << 21) >> 21;  // by0 - ay0
+    return wa != 0 && ha != 0 && wb != 0 && hb != 0 && dx < wa && dx + wb > 0 && dy < ha && dy + hb > 0;
+}
+
 // the w word of particle b's position record: its range code
 __device__ __forceinline__ uint32_t range_of(const DevWorld &w, int b) {
     return __float_as_uint(__ldg(reinterpret_cast<const float *>(w.pr + b) + 3));
@@ -840,6 +856,7 @@ void launch_reorder(const DevWorld &w, const DevWorld &spare, int block, cudaStr
 // the list's first word h0 (count and flags) and the slot word's NL_LIVE bit
 __device__ __forceinline__ void list_head(const DevWorld &w, int i, int16_t *h, int h0) {
     h[0] = (int16_t)h0;
+    w.cmask[i] = CM_STALE;  // the match word described the old list
     const uint32_t sm = w.smask[i];
     const uint32_t nsm = h0 != 0 ? (sm | NL_LIVE) : (sm & ~NL_LIVE);
     if (nsm != sm) w.smask[i] = nsm;
@@ -1219,6 +1236,14 @@ __device__ __forceinline__ void narrow_test(const DevWorld &w, int i, int b, flo
     accept_partner(w, b, __float_as_uint(pa.w), __float_as_uint(pb.w), nr);
 }
 
+// The match word cm of a particle's slots against its candidate list (bits
+// 1..15: candidates that own a slot; 17..31: of these, the ones whose slot
+// changes when the candidate is not accepted): whether a pass that accepts
+// the candidates `pass` leaves every slot as it is.
+__device__ __forceinline__ bool cm_unchanged(uint32_t cm, uint32_t pass) {
+    return (pass & ~cm) == 0u && ((cm >> 16) & ~pass) == 0u;
+}
+
 // entry k (0..15) of a candidate list held in two int4
 __device__ __forceinline__ int nl_entry(int4 a, int4 b, int k) {
     const int q = k >> 1;
@@ -1279,13 +1304,16 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
     }
     // the candidate list only when it is not empty, del_pos only for a
     // particle with contacts (its force loop reads it)
-    if (PART != 2 && (mask & NL_LIVE)) prefetch_l1(&w.nl[2 * (size_t)i]);
+    if (PART != 2 && (mask & NL_LIVE)) {
+        prefetch_l1(&w.nl[2 * (size_t)i]);
+        prefetch_l1(&w.cmask[i]);
+    }
     if (PART != 1 && (mask & ((1u << K) - 1u))) prefetch_l1(&w.dp[i]);
     const int N = w.N;
-    for (uint32_t left = mask & ((1u << K) - 1u); left; left &= left - 1) {
+    for (uint32_t left = PART != 1 ? mask & ((1u << K) - 1u) : 0u; left; left &= left - 1) {
         const int j = __ffs(left) - 1;
         prefetch_l1(&w.s_b[j * N + i]);
-        if (PART != 1) prefetch_l1(&w.s_tf[j * N + i]);
+        prefetch_l1(&w.s_tf[j * N + i]);
         if ((mask >> (BSHIFT + j)) & 1u) prefetch_l1(&w.s_bonded[j * N + i]);
     }
     const int s = (int)meta_scene(m);
@@ -1310,12 +1338,14 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
     if (detect) {                                                  // :126-228
         nr.cnt = 0;
         const uint32_t ca = __float_as_uint(pa.w);  // the particle's bucket range
-        bool direct = false;       // accepted partners that own a slot only mark it found
-        int n_acc = 0;             // partners accepted in direct mode
-        uint32_t found_slots = 0u;
         const int4 la = (mask & NL_LIVE) ? __ldg(&w.nl[2 * (size_t)i]) : make_int4(0, 0, 0, 0);
         const int h0 = la.x & 0xFFFF;
         const int lc = h0 & 0xFF;
+        // the match word (a particle with slots and no list: its slots are gone over)
+        const uint32_t cm = (mask & NL_LIVE) ? w.cmask[i] : (mask & ((1u << K) - 1u)) ? CM_STALE : 0u;
+        bool listed = false;       // partners come from the candidate list alone
+        int4 lb = make_int4(0, 0, 0, 0);
+        uint32_t pass = 0u;        // candidates (bits 1..15) the reference accepts
         if (lc == NL_BIG) {
             // a large particle: k_big_narrow left its partners, in order, in
             // the record of the particle's rank in its cell (list word 1)
@@ -1324,50 +1354,37 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
             for (int q = 0; q < n; ++q) nr_ci[q * IB + threadIdx.x] = acc_g[q];
             nr.cnt = n;
         } else if (lc != NL_OVERFLOW) {
-            const int4 lb = lc > 7 ? __ldg(&w.nl[2 * (size_t)i + 1]) : make_int4(0, 0, 0, 0);
-            // distance tests first, all gathers independent; then the bucket
-            // test and ordering of the partners that touch.  The unrolled
-            // tests stop at the longest list among the warp's lanes here
-            // (a warp-uniform exit: sparse warps skip the empty tail).
-            uint32_t pass = 0u;
+            if (lc > 7) lb = __ldg(&w.nl[2 * (size_t)i + 1]);
+            // distance and bucket tests, all gathers independent.  The
+            // unrolled tests stop at the longest list among the warp's lanes
+            // here (a warp-uniform exit: sparse warps skip the empty tail).
             const int lmax = __reduce_max_sync(__activemask(), lc);
 #pragma unroll
             for (int k = 1; k <= NL; ++k) {
                 if (k > lmax) break;
-                if (k <= lc && touching(pa, __ldg(&w.pr[i + nl_entry(la, lb, k)]))) pass |= 1u << k;
-            }
-            // With at most 14 partners touching and no large particle near,
-            // the accepted list is never cut at 14, so a partner that already
-            // owns a slot needs no key: it only marks the slot found.  The
-            // others are keyed and ordered for creation as usual.
-            direct = !(h0 & NL_NEAR_BIG) && __popc(pass) <= K;
-            if (direct) {
-                for (; pass; pass &= pass - 1) {
-                    const int b = i + nl_entry(la, lb, __ffs(pass) - 1);
-                    unsigned rank;
-                    if (!shared_bucket(w, ca, range_of(w, b), rank)) continue;
-                    ++n_acc;
-                    uint32_t hit = 0u;
-                    for (uint32_t left = mask & ((1u << K) - 1u); left; left &= left - 1) {
-                        const int j = __ffs(left) - 1;
-                        if (w.s_b[j * N + i] == b) hit |= 1u << j;
-                    }
-                    if (hit) {
-                        found_slots |= hit;
-                        continue;
-                    }
-                    top14_insert((rank << 28) | (uint32_t)__ldg(&w.orig[b]), b, nr);
+                if (k <= lc) {
+                    const float4 pb = __ldg(&w.pr[i + nl_entry(la, lb, k)]);
+                    if (touching(pa, pb) && shares_bucket(ca, __float_as_uint(pb.w))) pass |= 1u << k;
                 }
-            } else {
+            }
+            if (wide_range(ca)) {  // the range limits, checked on every partner
+                unsigned rank;
+                for (uint32_t q = pass; q; q &= q - 1)
+                    shared_bucket(w, ca, range_of(w, i + nl_entry(la, lb, __ffs(q) - 1)), rank);
+            }
+            // With at most 14 partners and no large particle near, the
+            // accepted list is never cut at 14.
+            listed = !(h0 & NL_NEAR_BIG) && __popc(pass) <= K;
+            if (!listed) {
                 for (; pass; pass &= pass - 1) {
                     const int b = i + nl_entry(la, lb, __ffs(pass) - 1);
                     accept_partner(w, b, ca, range_of(w, b), nr);
                 }
-            }
-            if (h0 & NL_NEAR_BIG) {
-                int bf, bn;
-                big_cell(w, P, bf, bn);
-                for (int k = 0; k < bn; ++k) narrow_test(w, i, w.sorted[bf + k], pa, nr);
+                if (h0 & NL_NEAR_BIG) {
+                    int bf, bn;
+                    big_cell(w, P, bf, bn);
+                    for (int k = 0; k < bn; ++k) narrow_test(w, i, w.sorted[bf + k], pa, nr);
+                }
             }
         } else {
             if (P.n_big > 0) {
@@ -1385,42 +1402,75 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
                 for (int k = beg; k < end; ++k) narrow_test(w, i, w.sorted[k], pa, nr);
             }
         }
-        const int cnt = nr.cnt;
         const int t = threadIdx.x;
-        if ((direct ? n_acc : cnt) == K) atomicAdd(&w.stats[0], 1ull);
-        // delete contacts that were not found (:185-204); `matched` marks the
-        // accepted partners that already own a slot
-        uint32_t matched = 0u;
-        for (uint32_t left = mask & ((1u << K) - 1u); left; left &= left - 1) {
-            const int j = __ffs(left) - 1;
-            bool found = (found_slots >> j) & 1u;
-            if (!direct) {
-                const int sb = w.s_b[j * N + i];
-                for (int q = 0; q < cnt; ++q) {
-                    const bool hit = nr_ci[q * IB + t] == sb;
-                    found |= hit;
-                    matched |= hit ? (1u << q) : 0u;
+        if ((listed ? __popc(pass) : nr.cnt) == K) atomicAdd(&w.stats[0], 1ull);
+        if (!listed || (cm & CM_STALE) != 0u || !cm_unchanged(cm, pass)) {
+            uint32_t found_slots = 0u;
+            if (listed) {
+                // a partner that already owns a slot marks it found; the
+                // others are keyed and ordered for creation
+                for (uint32_t q = pass; q; q &= q - 1) {
+                    const int b = i + nl_entry(la, lb, __ffs(q) - 1);
+                    uint32_t hit = 0u;
+                    for (uint32_t left = mask & ((1u << K) - 1u); left; left &= left - 1) {
+                        const int j = __ffs(left) - 1;
+                        if (w.s_b[j * N + i] == b) hit |= 1u << j;
+                    }
+                    if (hit) found_slots |= hit;
+                    else accept_partner(w, b, ca, range_of(w, b), nr);
                 }
             }
-            if (found) continue;
-            const bool bonded_nn = (mask >> (BSHIFT + j)) & 1u;   // bonded >= 0
-            if (!bonded_nn || bonds_model == 0) {
-                mask &= ~(1u << j);
-            } else if (bonds_model <= 1 && w.s_bonded[j * N + i] > 0) {
+            const int cnt = nr.cnt;
+            // delete contacts that were not found (:185-204); `matched` marks the
+            // accepted partners that already own a slot
+            uint32_t matched = 0u;
+            for (uint32_t left = mask & ((1u << K) - 1u); left; left &= left - 1) {
+                const int j = __ffs(left) - 1;
+                bool found = (found_slots >> j) & 1u;
+                if (!listed) {
+                    const int sb = w.s_b[j * N + i];
+                    for (int q = 0; q < cnt; ++q) {
+                        const bool hit = nr_ci[q * IB + t] == sb;
+                        found |= hit;
+                        matched |= hit ? (1u << q) : 0u;
+                    }
+                }
+                if (found) continue;
+                const bool bonded_nn = (mask >> (BSHIFT + j)) & 1u;   // bonded >= 0
+                if (!bonded_nn || bonds_model == 0) {
+                    mask &= ~(1u << j);
+                } else if (bonds_model <= 1 && w.s_bonded[j * N + i] > 0) {
+                    w.s_tf[j * N + i] = 0.0f;
+                }
+            }
+            // create new contacts in the last empty slot (:207-227); a deleted
+            // slot never holds an accepted partner, so `matched` is the
+            // reference's "existing" test
+            for (int q = 0; q < cnt; ++q) {
+                if ((matched >> q) & 1u) continue;
+                const uint32_t empty = (~mask) & ((1u << K) - 1u);
+                if (empty == 0u) continue;
+                const int j = 31 - __clz(empty);
+                mask |= 1u << j;
+                w.s_b[j * N + i] = nr_ci[q * IB + t];
                 w.s_tf[j * N + i] = 0.0f;
             }
-        }
-        // create new contacts in the last empty slot (:207-227); a deleted
-        // slot never holds an accepted partner, so `matched` is the
-        // reference's "existing" test
-        for (int q = 0; q < cnt; ++q) {
-            if ((matched >> q) & 1u) continue;
-            const uint32_t empty = (~mask) & ((1u << K) - 1u);
-            if (empty == 0u) continue;
-            const int j = 31 - __clz(empty);
-            mask |= 1u << j;
-            w.s_b[j * N + i] = nr_ci[q * IB + t];
-            w.s_tf[j * N + i] = 0.0f;
+            // the match word of the slots as they are now
+            if (mask & NL_LIVE) {
+                uint32_t next = CM_STALE;
+                if (listed && bonds_model != 1) {
+                    next = 0u;
+                    for (uint32_t left = mask & ((1u << K) - 1u); left; left &= left - 1) {
+                        const int j = __ffs(left) - 1;
+                        const int off = w.s_b[j * N + i] - i;
+                        uint32_t at = 0u;
+                        for (int k = 1; k <= lc; ++k) at |= nl_entry(la, lb, k) == off ? 1u << k : 0u;
+                        next |= at;
+                        if (bonds_model == 0 || !((mask >> (BSHIFT + j)) & 1u)) next |= at << 16;
+                    }
+                }
+                if (next != cm) w.cmask[i] = next;
+            }
         }
     }
 
@@ -1657,7 +1707,11 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
         if (!(zero && (mask & DF_ZERO))) w.dF[i] = make_float4(acc.d0, acc.d1, acc.d2, 0.0f);
         mask = zero ? (mask | DF_ZERO) : (mask & ~DF_ZERO);
     }
-    if (mask != before) w.smask[i] = mask;
+    if (mask != before) {
+        w.smask[i] = mask;
+        // a bond broke: its slot is a plain contact from now on
+        if (((mask ^ before) & ~mask & BONDED_BITS) != 0u) w.cmask[i] = CM_STALE;
+    }
 }
 
 // End of step, run by the last warp of k_interact or by k_end_step's block: breaks of this step

@@ -36,6 +36,8 @@ constexpr int K = DEM_MAX_CONTACTS;
 constexpr int BSHIFT = 16;  // first bonded-field bit of the slot word
 constexpr uint32_t DF_ZERO = 1u << 31;  // slot-word bit: dF holds +0, +0, +0
 constexpr uint32_t NL_LIVE = 1u << 14;  // slot-word bit: the candidate list is not empty
+constexpr uint32_t BONDED_BITS = ((1u << K) - 1u) << BSHIFT;
+constexpr uint32_t CM_STALE = 1u;       // match word: nothing is known (see DevWorld::cmask)
 
 // meta word: fixity predicates, external-force flag, material, scene
 enum : uint32_t {
@@ -158,6 +160,12 @@ struct DevWorld {
     int32_t *err;
     // candidate lists (built at rebuilds)
     int4 *nl;                   // [N][2] candidate lists (see NL)
+    // Match word of each particle's slots against its candidate list: bits
+    // 1..15 the candidates that own a slot, bits 17..31 those of them whose
+    // slot is changed by a pass that does not accept the candidate (the
+    // unbonded ones, and all under bond model 0); CM_STALE when the list is
+    // new or the word does not apply (bond model 1, a large particle near).
+    uint32_t *cmask;
     float2 *pbuild;             // [N] position at the last rebuild
     uint32_t *kbuild;           // [N] search cell at the last rebuild
     int32_t *rebuild;           // 1 = the next rebuild body runs

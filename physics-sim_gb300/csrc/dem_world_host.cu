@@ -506,6 +506,7 @@ int World::alloc(int N, int C, int B, int S, int M, int MP, int TB, uint32_t ev_
     w.step = dalloc<long long>(owned, 1, ok);
     w.err = dalloc<int32_t>(owned, 1, ok);
     w.nl = dalloc<int4>(owned, 2 * (size_t)N, ok);
+    w.cmask = dalloc<uint32_t>(owned, N, ok);
     w.pbuild = dalloc<float2>(owned, N, ok);
     w.kbuild = dalloc<uint32_t>(owned, N, ok);
     w.rebuild = dalloc<int32_t>(owned, 1, ok);
@@ -1496,6 +1497,11 @@ int World::set_params(int s, const dem_params &p) {
     h.cc2_0 = cc[2];
     int rc = push_par(s);
     if (rc) return rc;
+    if (old.bonds != p.bonds && h.n > 0) {
+        // the match words depend on the bond model: all stale
+        static_assert(CM_STALE == 1u, "the memset below sets the bit");
+        CK(cudaMemsetAsync(d.cmask + h.particle_base, 0xFF, 4 * (size_t)h.n, stream));
+    }
     rc = push_det();
     if (rc) return rc;
     update_kernel_form();
@@ -1809,9 +1815,24 @@ void World::update_param_source() {
     std::memcpy(&par_pv, &kp, sizeof(ScenePar));
 }
 
+// One Simulation kernel or two.  Where particles have many contacts and some
+// are bonded, the single kernel's register cap spills inside the force loop
+// and the split pays (4.2 M-particle impact bed 469 -> 395 us a step, its
+// 262,145-particle crop 68 -> 62); without bonds, or with fewer contacts a
+// particle, the second read of the records costs more (1 M-particle bed 94.5
+// against 98.5 us, 128 scenes of the mix 124 against 131), and served worlds,
+// whose scenes come and go, would capture their graphs anew at each change.
+void World::update_split() {
+    const int want = split_narrow || (free_slot < 0 && kernel_form != 0 && dense_cells()) ? 1 : 0;
+    if (want == d.split) return;
+    d.split = want;
+    drop_graph();
+}
+
 int World::step(int n_steps) {
     if (n_steps < 0) return fail(DEM_E_INVALID, "n_steps < 0");
     update_param_source();
+    update_split();
     int k = 0;
     if (use_graphs && !timing && n_steps > 0) {
         if (par_ps != graph_ps || std::memcmp(&par_pv, &graph_par, sizeof(ScenePar)) != 0) {

@@ -200,6 +200,7 @@ class World {
     int par_ps = PS_SCENE;
     ScenePar par_pv{};
     void update_param_source();
+    void update_split();
     int graph_ps = -1;
     ScenePar graph_par{};
     int parity = 0;                    // which pr/dp/rr buffers are current
