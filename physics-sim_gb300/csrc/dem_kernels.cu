@@ -98,11 +98,6 @@ __device__ __forceinline__ bool shares_bucket(uint32_t ca, uint32_t cb) {
     return wa != 0 && ha != 0 && wb != 0 && hb != 0 && dx < wa && dx + wb > 0 && dy < ha && dy + hb > 0;
 }
 
-// the w word of particle b's position record: its range code
-__device__ __forceinline__ uint32_t range_of(const DevWorld &w, int b) {
-    return __float_as_uint(__ldg(reinterpret_cast<const float *>(w.pr + b) + 3));
-}
-
 // search-grid cell of a position (floor, clamped to the grid)
 __device__ __forceinline__ void search_xy(const ScenePar &P, float x, float y, int &cx, int &cy) {
     int a = __float2int_rd((x - P.g_x0) * P.g_inv);
@@ -254,22 +249,20 @@ __device__ __forceinline__ bool last_warp(uint32_t *ticket) {
 // for a rebuild before this step's Simulation pass.
 // 2D_LOM.wgsl:85-152 of one particle from its records (p, v, a, flags m,
 // rebuild position b); `ext`: positions were set externally, so the
-// displacement is the stored dext.  Position and bucket range go to pr_out,
-// the displacement to dp_out, the velocities and rotation to vw, and
-// data[4..6] to d4 when keep_d4 (a later LOM pass of the same call would
-// overwrite it).
+// displacement is the stored dext.  Leaves the new position and bucket range
+// in p, the velocities and rotation in v, the displacement in d, data[4..6]
+// in d4, and in `moved` whether the candidate lists no longer hold.
 // U: the scene's settings (P.p) and model constants, P its geometry; the
 // two are the same record unless the world's scenes share the former.
-__device__ __forceinline__ void lom_core(const DevWorld &w, const ScenePar &P, const ScenePar &U, int i,
-                                         uint32_t m, float4 p, float4 v, float4 a, float2 b, bool ext, float4 dext,
-                                         bool keep_d4, float4 *pr_out, float4 *dp_out) {
+__device__ __forceinline__ void lom_core(const ScenePar &P, const ScenePar &U, uint32_t m, float4 &p, float4 &v,
+                                         float4 a, float2 b, bool ext, float4 dext, float4 &d, float4 &d4,
+                                         bool &moved) {
     const float dT = U.p.dT;
     float ivx = v.x, ivy = v.y, iw = v.z;
     if (m & M_KICK_X) ivx = ivx + (a.x * dT) * 0.5f;               // :88
     if (m & M_KICK_Y) ivy = ivy + (a.y * dT) * 0.5f;               // :89
     if (m & M_KICK_R) iw = iw + (a.z * dT) * 0.5f;                 // :90
-    if (keep_d4) w.d4[i] = make_float4(ivx, ivy, iw, 0.0f);        // :92-94
-    float4 d;
+    d4 = make_float4(ivx, ivy, iw, 0.0f);                          // :92-94
     if (!ext) {                                                    // :96-99
         d = make_float4(ivx * dT, ivy * dT, iw * dT, 0.0f);
     } else {
@@ -322,18 +315,16 @@ __device__ __forceinline__ void lom_core(const DevWorld &w, const ScenePar &P, c
         ref_range(P, p.x, p.y, p.z, x0, x1, y0, y1);
         p.w = range_code(x0, x1, y0, y1);
     }
-    pr_out[i] = p;
-    w.vw[i] = make_float4(ivx, ivy, iw, rot);                      // :151-152
-    if (!ext) dp_out[i] = d;
+    v = make_float4(ivx, ivy, iw, rot);                            // :151-152
     const float ex = p.x - b.x, ey = p.y - b.y;
-    if (!(ex * ex + ey * ey <= P.disp_limit2)) atomicOr(w.rebuild, 1);
+    moved = !(ex * ex + ey * ey <= P.disp_limit2);
 }
 
 __device__ __forceinline__ void lom_particle(const DevWorld &w, int i) {
     // all of the particle's records requested at once (valid for any i < N)
     const uint32_t m = w.meta[i];
-    const float4 p = w.pr[i];
-    const float4 v = w.vw[i];
+    float4 p = w.pr[i];
+    float4 v = w.vw[i];
     const float4 a = w.ac[i];
     const float2 b = w.pbuild[i];
     const int s = (int)meta_scene(m);
@@ -341,12 +332,16 @@ __device__ __forceinline__ void lom_particle(const DevWorld &w, int i) {
     const ScenePar &P = w.par[s];
     if (p.z == 0.0f) return;                                       // :83
     const bool ext = w.cc3[s] != 0;
-    lom_core(w, P, P, i, m, p, v, a, b, ext, ext ? w.dp[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f), true, w.pr, w.dp);
+    float4 d, d4;
+    bool moved;
+    lom_core(P, P, m, p, v, a, b, ext, ext ? w.dp[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f), d, d4, moved);
+    w.d4[i] = d4;
+    w.pr[i] = p;
+    w.vw[i] = v;
+    if (!ext) w.dp[i] = d;
+    if (moved) atomicOr(w.rebuild, 1);
 }
 
-// With w.ticket the kernel's last warp sets the rebuild conditional; without
-// it (large worlds, where thousands of fenced ticket atomics cost more than a
-// launch) k_decide does it.
 // a 128-particle chunk holding at least one particle of a scene (served
 // worlds keep the map; elsewhere every chunk is live).  Warps never straddle
 // chunks, so the test is warp-uniform.
@@ -354,6 +349,10 @@ __device__ __forceinline__ bool chunk_live(const DevWorld &w, int i) {
     return w.live == nullptr || __ldg(&w.live[i >> 7]) != 0;
 }
 
+#ifndef DEM_STEP_DEVICE_CODE  // dem_steps.cu includes this file for the step's device functions alone
+// With w.ticket the kernel's last warp sets the rebuild conditional; without
+// it (large worlds, where thousands of fenced ticket atomics cost more than a
+// launch) k_decide does it.
 __global__ void __launch_bounds__(PK_MAX_THREADS) k_lom(DevWorld w, int in_graph, cudaGraphConditionalHandle cond) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < w.N && chunk_live(w, i)) lom_particle(w, i);
@@ -428,7 +427,7 @@ static int resident_blocks(const void *fn, int block) {
 }
 
 // SMs of the current device (cached per device)
-static int device_sms() {
+int device_sms() {
     static std::mutex mu;
     static std::vector<std::pair<int, int>> cache;  // device, SMs
     int dev = 0;
@@ -1135,6 +1134,8 @@ __global__ void __launch_bounds__(LT_THREADS) k_list_tiles(DevWorld w, const int
 __global__ void k_rebuild_done(DevWorld w, const int32_t *gate) {
     if (gated_off(gate)) return;
     *w.rebuild = 0;
+    clear_run_barrier(*w.run);
+    w.run->linked = 0;
     const unsigned long long n = w.stats[4] + 1ull;
     w.stats[4] = n;
     // the next rebuild reorders when it is the first of a new group of reorder_every
@@ -1164,6 +1165,8 @@ int launch_list_build(const DevWorld &w, int block, cudaStream_t st, const int32
     return staged ? 3 : 2;
 }
 
+#endif  // DEM_STEP_DEVICE_CODE
+
 // -------------------------------------------------------------- interact
 // 2D_Simulation.wgsl:108-262 per particle.
 //
@@ -1180,25 +1183,28 @@ constexpr int IB = 128;  // threads per k_interact block
 
 // The accepted partners of one thread, kept sorted by (first shared bucket,
 // particle index) in shared memory (slot-major, so a warp's accesses fall in
-// distinct banks): key = rank << 28 | scene-local index.
-__shared__ uint32_t nr_ck[K * IB];  // [K][IB] sort keys of the accepted partners
-__shared__ int nr_ci[K * IB];       // [K][IB] their internal indices
-
+// distinct banks): key = rank << 28 | scene-local index.  ck and ci point at
+// the thread's column of two [K][ST] arrays: sort keys and internal indices.
+template <int ST>
 struct Narrow {
-    int cnt;
+    uint32_t *ck;
+    int *ci;
+    int cnt = 0;
+    __device__ __forceinline__ uint32_t &key(int q) { return ck[q * ST]; }
+    __device__ __forceinline__ int &idx(int q) { return ci[q * ST]; }
 };
 
-__device__ __forceinline__ void top14_insert(uint32_t key, int idx, Narrow &nr) {
-    const int t = threadIdx.x;
-    if (nr.cnt == K && key >= nr_ck[(K - 1) * IB + t]) return;
+template <int ST>
+__device__ __forceinline__ void top14_insert(uint32_t key, int idx, Narrow<ST> &nr) {
+    if (nr.cnt == K && key >= nr.key(K - 1)) return;
     int pos = nr.cnt < K ? nr.cnt : K - 1;
-    while (pos > 0 && nr_ck[(pos - 1) * IB + t] > key) {
-        nr_ck[pos * IB + t] = nr_ck[(pos - 1) * IB + t];
-        nr_ci[pos * IB + t] = nr_ci[(pos - 1) * IB + t];
+    while (pos > 0 && nr.key(pos - 1) > key) {
+        nr.key(pos) = nr.key(pos - 1);
+        nr.idx(pos) = nr.idx(pos - 1);
         --pos;
     }
-    nr_ck[pos * IB + t] = key;
-    nr_ci[pos * IB + t] = idx;
+    nr.key(pos) = key;
+    nr.idx(pos) = idx;
     if (nr.cnt < K) ++nr.cnt;
 }
 
@@ -1222,18 +1228,20 @@ __device__ __forceinline__ bool touching(float4 pa, float4 pb) {
 // b (range code cb) passed the distance test: keep it when its AABB shares a
 // reference bucket with the particle's (range code ca), keyed by the first
 // shared bucket
-__device__ __forceinline__ void accept_partner(const DevWorld &w, int b, uint32_t ca, uint32_t cb, Narrow &nr) {
+template <int ST>
+__device__ __forceinline__ void accept_partner(const DevWorld &w, int b, uint32_t ca, uint32_t cb, Narrow<ST> &nr) {
     unsigned rank;
     if (!shared_bucket(w, ca, cb, rank)) return;
     const uint32_t key = (rank << 28) | (uint32_t)__ldg(&w.orig[b]);
     top14_insert(key, b, nr);
 }
 
-__device__ __forceinline__ void narrow_test(const DevWorld &w, int i, int b, float4 pa, Narrow &nr) {
+template <class Own, int ST>
+__device__ __forceinline__ void narrow_test(const DevWorld &w, int i, int b, const Own &o, Narrow<ST> &nr) {
     if (b == i) return;
-    const float4 pb = __ldg(&w.pr[b]);
-    if (!touching(pa, pb)) return;
-    accept_partner(w, b, __float_as_uint(pa.w), __float_as_uint(pb.w), nr);
+    const float4 pb = o.partner(w, b);
+    if (!touching(o.pa, pb)) return;
+    accept_partner(w, b, __float_as_uint(o.pa.w), __float_as_uint(pb.w), nr);
 }
 
 // The match word cm of a particle's slots against its candidate list (bits
@@ -1252,11 +1260,137 @@ __device__ __forceinline__ int nl_entry(int4 a, int4 b, int k) {
     return (k & 1) ? (v >> 16) : (int)(int16_t)(v & 0xFFFF);
 }
 
+// the entry (1..15) of a candidate list that holds the offset off, 0 when
+// none does: two entries a word compared at once.  Offsets are never 0 and
+// an unused entry may hold an old offset, so the count (entry 0, low byte)
+// bounds the answer.
+__device__ __forceinline__ int nl_find(int4 a, int4 b, int off) {
+    if (off < -32768 || off > 32767) return 0;
+    const uint32_t two = (uint32_t)(off & 0xFFFF) * 0x10001u;
+    const int v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t eq = 0u;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const uint32_t x = (uint32_t)v[q] ^ two;
+        if ((x & 0xFFFFu) == 0u) eq |= 1u << (2 * q);
+        if ((x >> 16) == 0u) eq |= 2u << (2 * q);
+    }
+    eq &= (2u << (a.x & 0xFF)) - 2u;  // entries 1..count
+    return eq ? __ffs(eq) - 1 : 0;
+}
+
 // L1 prefetch of one line (sm_90+ PTX): the later load of the same address
 // finds it on chip instead of waiting a DRAM round trip then.
 __device__ __forceinline__ void prefetch_l1(const void *p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
+
+// The particle's own state and the way to its partners' records, for
+// interact_particle.  HbmOwn: everything in device memory, a launch a step.
+// The particle's own records: the ones needed first are loaded now, the
+// rest (read only after the scene, detection and slot checks resolve) are
+// prefetched now, so the DRAM round trips overlap instead of following one
+// another.
+template <int PART, bool FUSE>
+struct HbmOwn {
+    static constexpr bool RESIDENT = false;
+    uint32_t m, mask;
+    float4 pa;
+    int N, i;
+    __device__ __forceinline__ HbmOwn(const DevWorld &w, int i_) : N(w.N), i(i_) {
+        m = w.meta[i];
+        pa = w.pr[i];
+        mask = w.smask[i];
+        if (PART != 1) {
+            prefetch_l1(&w.vw[i]);
+            if (FUSE) prefetch_l1(&w.pbuild[i]);
+        }
+        // the candidate list only when it is not empty, del_pos only for a
+        // particle with contacts (its force loop reads it)
+        if (PART != 2 && (mask & NL_LIVE)) {
+            prefetch_l1(&w.nl[2 * (size_t)i]);
+            prefetch_l1(&w.cmask[i]);
+        }
+        if (PART != 1 && (mask & SLOT_BITS)) prefetch_l1(&w.dp[i]);
+        for (uint32_t left = PART != 1 ? mask & SLOT_BITS : 0u; left; left &= left - 1) {
+            const int j = __ffs(left) - 1;
+            prefetch_l1(&w.s_b[j * N + i]);
+            prefetch_l1(&w.s_tf[j * N + i]);
+            if ((mask >> (BSHIFT + j)) & 1u) prefetch_l1(&w.s_bonded[j * N + i]);
+        }
+    }
+    __device__ __forceinline__ const ScenePar &scene(const DevWorld &w, int s) const { return w.par[s]; }
+    __device__ __forceinline__ bool acts(const DevWorld &w, int s) const { return w.act[s] != 0; }
+    __device__ __forceinline__ bool detects(const DevWorld &w, int s) const { return w.det[s] != 0; }
+    __device__ __forceinline__ long long left(const DevWorld &w, int s) const { return w.remaining[s]; }
+    __device__ __forceinline__ long long step(const DevWorld &w) const { return *w.step; }
+    // candidate list and match word
+    __device__ __forceinline__ int4 list(const DevWorld &w, int h) const { return __ldg(&w.nl[2 * (size_t)i + h]); }
+    __device__ __forceinline__ uint32_t match(const DevWorld &w) const { return w.cmask[i]; }
+    __device__ __forceinline__ void set_match(const DevWorld &w, uint32_t c) { w.cmask[i] = c; }
+    __device__ __forceinline__ uint64_t slot_candidates() const { return 0u; }
+    template <int ST>
+    __device__ __forceinline__ bool search_cells(const DevWorld &, int, Narrow<ST> &) const { return false; }
+    __device__ __forceinline__ void set_slot_candidates(uint64_t) {}
+    // slots
+    __device__ __forceinline__ int slot_b(const DevWorld &w, int j) const { return w.s_b[j * N + i]; }
+    __device__ __forceinline__ int slot_bonded(const DevWorld &w, int j) const { return w.s_bonded[j * N + i]; }
+    __device__ __forceinline__ float slot_tf(const DevWorld &w, int j) const { return w.s_tf[j * N + i]; }
+    __device__ __forceinline__ float slot_btf(const DevWorld &w, int j) const { return w.s_btf[j * N + i]; }
+    __device__ __forceinline__ float slot_thb(const DevWorld &w, int j) const { return w.s_thb[j * N + i]; }
+    __device__ __forceinline__ void new_slot(const DevWorld &w, int j, int b) {
+        w.s_b[j * N + i] = b;
+        w.s_tf[j * N + i] = 0.0f;
+    }
+    __device__ __forceinline__ void set_bonded(const DevWorld &w, int j, int x) { w.s_bonded[j * N + i] = x; }
+    __device__ __forceinline__ void set_tf(const DevWorld &w, int j, float x) { w.s_tf[j * N + i] = x; }
+    __device__ __forceinline__ void set_btf(const DevWorld &w, int j, float x) { w.s_btf[j * N + i] = x; }
+    __device__ __forceinline__ void set_thb(const DevWorld &w, int j, float x) { w.s_thb[j * N + i] = x; }
+    __device__ __forceinline__ void set_mask(const DevWorld &w, uint32_t x, uint32_t before) {
+        if (x != before) w.smask[i] = x;
+    }
+    // partners
+    __device__ __forceinline__ float4 partner(const DevWorld &w, int b) const { return __ldg(&w.pr[b]); }
+    __device__ __forceinline__ uint32_t partner_range(const DevWorld &w, int b) const {
+        return __float_as_uint(__ldg(reinterpret_cast<const float *>(w.pr + b) + 3));
+    }
+    __device__ __forceinline__ float4 partner_disp(const DevWorld &w, int b) const { return __ldg(&w.dp[b]); }
+    __device__ __forceinline__ int bond_status(const DevWorld &w, int g) const { return w.b_status[g]; }
+    __device__ __forceinline__ void broke() {}
+    __device__ __forceinline__ void record(const DevWorld &, float4, float, float, float, float) {}
+    // the rest of the particle's own record
+    __device__ __forceinline__ float2 stiffness(const DevWorld &w, int, int at) const { return __ldg(&w.pair[at]); }
+    __device__ __forceinline__ float density(const DevWorld &w, int at) const { return w.mats[at].density; }
+    __device__ __forceinline__ float4 external(const DevWorld &w) const { return w.fx[i]; }
+    __device__ __forceinline__ float4 disp(const DevWorld &w) const { return w.dp[i]; }
+    __device__ __forceinline__ float4 vel(const DevWorld &w) const { return w.vw[i]; }
+    __device__ __forceinline__ float2 rebuilt_at(const DevWorld &w) const { return w.pbuild[i]; }
+    __device__ __forceinline__ void set_vel(const DevWorld &w, float4 v) { w.vw[i] = v; }
+    // the next step's position and displacement (and, when keep_d4, its data[4..6])
+    __device__ __forceinline__ void advance(const DevWorld &w, float4 p, float4 v, float4 d, float4 d4, bool moved,
+                                            bool keep_d4) {
+        if (keep_d4) w.d4[i] = d4;
+        w.pr_n[i] = p;
+        w.vw[i] = v;
+        w.dp_n[i] = d;
+        if (moved) atomicOr(w.rebuild, 1);
+    }
+    // the particle does not step on: its record crosses to the other buffers
+    __device__ __forceinline__ void stay(const DevWorld &w) {
+        w.pr_n[i] = pa;
+        w.dp_n[i] = w.dp[i];
+    }
+};
+
+// what the force loop reads of one slot: the slot's fields, then what they index
+struct SlotIn {
+    bool bnn;
+    int b, bonded, st;
+    float tf, btf, thb, blen;
+    float4 pb, db;
+    uint32_t mb;
+    float2 str;
+};
 
 // The Simulation pass of one particle.  PART selects what runs: 0 all of it
 // (k_interact), 1 the narrow phase and slot bookkeeping (k_narrow), 2 the
@@ -1288,61 +1422,71 @@ __device__ __forceinline__ void prefetch_l1(const void *p) {
 // constants (the fields read through U) come with the launch, the rest from
 // w.par[scene].  Every field read through U is one that shared_settings
 // (dem_world.cuh) copies (tests/test_param_source.py checks this source).
-template <int PART, bool FUSE, int FORM, int PS>
-__device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narrow &nr, bool lom_final,
+template <int PART, bool FUSE, int FORM, int PS, class Own, int ST>
+__device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Own &o, Narrow<ST> &nr, bool lom_final,
                                                   const ScenePar &Pv) {
-    // The particle's own records: the ones needed first are loaded now, the
-    // rest (read only after the scene, detection and slot checks resolve)
-    // are prefetched now, so the DRAM round trips overlap instead of
-    // following one another.
-    const uint32_t m = w.meta[i];
-    const float4 pa = w.pr[i];
-    uint32_t mask = w.smask[i];
-    if (PART != 1) {
-        prefetch_l1(&w.vw[i]);
-        if (FUSE) prefetch_l1(&w.pbuild[i]);
-    }
-    // the candidate list only when it is not empty, del_pos only for a
-    // particle with contacts (its force loop reads it)
-    if (PART != 2 && (mask & NL_LIVE)) {
-        prefetch_l1(&w.nl[2 * (size_t)i]);
-        prefetch_l1(&w.cmask[i]);
-    }
-    if (PART != 1 && (mask & ((1u << K) - 1u))) prefetch_l1(&w.dp[i]);
-    const int N = w.N;
-    for (uint32_t left = PART != 1 ? mask & ((1u << K) - 1u) : 0u; left; left &= left - 1) {
-        const int j = __ffs(left) - 1;
-        prefetch_l1(&w.s_b[j * N + i]);
-        prefetch_l1(&w.s_tf[j * N + i]);
-        if ((mask >> (BSHIFT + j)) & 1u) prefetch_l1(&w.s_bonded[j * N + i]);
-    }
+    const uint32_t m = o.m;
+    const float4 pa = o.pa;
+    uint32_t mask = o.mask;
     const int s = (int)meta_scene(m);
-    if (!w.act[s]) return;
-    const ScenePar &P = PS == PS_ONE ? Pv : w.par[s];
+    if (!o.acts(w, s)) return;
+    const ScenePar &P = PS == PS_ONE ? Pv : o.scene(w, s);
     const ScenePar &U = PS == PS_SCENE ? P : Pv;
     if (pa.z == 0.0f) {                                            // :113-118
         if (PART != 1) w.dF[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (FUSE) {
-            w.pr_n[i] = pa;
-            w.dp_n[i] = w.dp[i];
-        }
+        if (Own::RESIDENT) o.record(w, pa, o.vel(w).w, 0.0f, 0.0f, 0.0f);
+        if (FUSE) o.stay(w);
         return;
     }
     const uint32_t before = mask;
     const int bonds_model = FORM == 0 ? 0 : FORM == 3 ? 3 : U.p.bonds;
     constexpr bool MAY_F64 = FORM == -1;
 
+    const auto fetch = [&](int j) {
+        SlotIn q;
+        q.bnn = (mask >> (BSHIFT + j)) & 1u;                       // bonded >= 0
+        q.b = o.slot_b(w, j);
+        q.tf = o.slot_tf(w, j);
+        q.bonded = -1;                                             // any negative value acts alike
+        q.btf = q.thb = 0.0f;
+        if (q.bnn) {
+            q.bonded = o.slot_bonded(w, j);
+            if (bonds_model == 3) {
+                q.btf = o.slot_btf(w, j);
+                q.thb = o.slot_thb(w, j);
+            }
+        }
+        q.pb = o.partner(w, q.b);
+        q.db = o.partner_disp(w, q.b);
+        q.mb = U.n_mat == 1 ? 0u : __ldg(&w.meta[q.b]);
+        q.st = 0;
+        q.blen = 0.0f;
+        q.str = make_float2(U.p.bond_normal_strength, U.p.bond_shear_strength);
+        if (q.bnn) {
+            const int bg = P.bond_base + q.bonded;
+            q.st = o.bond_status(w, bg);
+            q.blen = w.b_length[bg];
+            if (U.has_strength) q.str = w.b_str[bg];
+        }
+        return q;
+    };
+    // a resident particle's slots are fetched one ahead; the first before the
+    // narrow phase, which seldom changes a slot
+    SlotIn ahead;
+    bool changed = false;
+    if (Own::RESIDENT && (mask & SLOT_BITS)) ahead = fetch(__ffs(mask & SLOT_BITS) - 1);
+
     // Loads that only some particles need (the bucket range, the second half
     // of the candidate list, del_pos) wait until the particle needs them.
-    const bool detect = PART != 2 && U.p.collisions == 1 && w.det[s] != 0;
+    const bool detect = PART != 2 && U.p.collisions == 1 && o.detects(w, s);
     if (detect) {                                                  // :126-228
         nr.cnt = 0;
         const uint32_t ca = __float_as_uint(pa.w);  // the particle's bucket range
-        const int4 la = (mask & NL_LIVE) ? __ldg(&w.nl[2 * (size_t)i]) : make_int4(0, 0, 0, 0);
+        const int4 la = (mask & NL_LIVE) ? o.list(w, 0) : make_int4(0, 0, 0, 0);
         const int h0 = la.x & 0xFFFF;
         const int lc = h0 & 0xFF;
         // the match word (a particle with slots and no list: its slots are gone over)
-        const uint32_t cm = (mask & NL_LIVE) ? w.cmask[i] : (mask & ((1u << K) - 1u)) ? CM_STALE : 0u;
+        const uint32_t cm = (mask & NL_LIVE) ? o.match(w) : (mask & SLOT_BITS) ? CM_STALE : 0u;
         bool listed = false;       // partners come from the candidate list alone
         int4 lb = make_int4(0, 0, 0, 0);
         uint32_t pass = 0u;        // candidates (bits 1..15) the reference accepts
@@ -1351,26 +1495,46 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
             // the record of the particle's rank in its cell (list word 1)
             const int32_t *acc_g = w.big_acc + 16 * (size_t)(P.big_base + la.y);
             const int n = acc_g[15];
-            for (int q = 0; q < n; ++q) nr_ci[q * IB + threadIdx.x] = acc_g[q];
+            for (int q = 0; q < n; ++q) nr.idx(q) = acc_g[q];
             nr.cnt = n;
         } else if (lc != NL_OVERFLOW) {
-            if (lc > 7) lb = __ldg(&w.nl[2 * (size_t)i + 1]);
+            if (lc > 7) lb = o.list(w, 1);
             // distance and bucket tests, all gathers independent.  The
             // unrolled tests stop at the longest list among the warp's lanes
             // here (a warp-uniform exit: sparse warps skip the empty tail).
             const int lmax = __reduce_max_sync(__activemask(), lc);
+            if (Own::RESIDENT) {
+                // few warps hide a gather's latency here: half a list in flight at once
 #pragma unroll
-            for (int k = 1; k <= NL; ++k) {
-                if (k > lmax) break;
-                if (k <= lc) {
-                    const float4 pb = __ldg(&w.pr[i + nl_entry(la, lb, k)]);
-                    if (touching(pa, pb) && shares_bucket(ca, __float_as_uint(pb.w))) pass |= 1u << k;
+                for (int h = 0; h < 2; ++h) {
+                    if (8 * h > lmax) break;
+                    float4 pb[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const int k = 8 * h + q;
+                        if (k > 0 && k <= lc) pb[q] = o.partner(w, i + nl_entry(la, lb, k));
+                    }
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const int k = 8 * h + q;
+                        if (k > 0 && k <= lc && touching(pa, pb[q]) && shares_bucket(ca, __float_as_uint(pb[q].w)))
+                            pass |= 1u << k;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int k = 1; k <= NL; ++k) {
+                    if (k > lmax) break;
+                    if (k <= lc) {
+                        const float4 pb = o.partner(w, i + nl_entry(la, lb, k));
+                        if (touching(pa, pb) && shares_bucket(ca, __float_as_uint(pb.w))) pass |= 1u << k;
+                    }
                 }
             }
             if (wide_range(ca)) {  // the range limits, checked on every partner
                 unsigned rank;
                 for (uint32_t q = pass; q; q &= q - 1)
-                    shared_bucket(w, ca, range_of(w, i + nl_entry(la, lb, __ffs(q) - 1)), rank);
+                    shared_bucket(w, ca, o.partner_range(w, i + nl_entry(la, lb, __ffs(q) - 1)), rank);
             }
             // With at most 14 partners and no large particle near, the
             // accepted list is never cut at 14.
@@ -1378,104 +1542,132 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
             if (!listed) {
                 for (; pass; pass &= pass - 1) {
                     const int b = i + nl_entry(la, lb, __ffs(pass) - 1);
-                    accept_partner(w, b, ca, range_of(w, b), nr);
+                    accept_partner(w, b, ca, o.partner_range(w, b), nr);
                 }
                 if (h0 & NL_NEAR_BIG) {
                     int bf, bn;
                     big_cell(w, P, bf, bn);
-                    for (int k = 0; k < bn; ++k) narrow_test(w, i, w.sorted[bf + k], pa, nr);
+                    for (int k = 0; k < bn; ++k) narrow_test(w, i, w.sorted[bf + k], o, nr);
                 }
             }
         } else {
             if (P.n_big > 0) {
                 int bf, bn;
                 big_cell(w, P, bf, bn);
-                for (int k = 0; k < bn; ++k) narrow_test(w, i, w.sorted[bf + k], pa, nr);
+                for (int k = 0; k < bn; ++k) narrow_test(w, i, w.sorted[bf + k], o, nr);
             }
-            const int local = (int)w.kbuild[i] - P.cell_base;
-            const int gx = local % P.g_w, gy = local / P.g_w;
-            const int cy0 = max(gy - P.stencil, 0), cy1 = min(gy + P.stencil, P.g_h - 1);
-            const int cx0 = max(gx - P.stencil, 0), cx1 = min(gx + P.stencil, P.g_w - 1);
-            for (int cy = cy0; cy <= cy1; ++cy) {
-                const int row = P.cell_base + cy * P.g_w;
-                const int beg = w.cell_start[row + cx0], end = w.cell_start[row + cx1 + 1];
-                for (int k = beg; k < end; ++k) narrow_test(w, i, w.sorted[k], pa, nr);
-            }
-        }
-        const int t = threadIdx.x;
-        if ((listed ? __popc(pass) : nr.cnt) == K) atomicAdd(&w.stats[0], 1ull);
-        if (!listed || (cm & CM_STALE) != 0u || !cm_unchanged(cm, pass)) {
-            uint32_t found_slots = 0u;
-            if (listed) {
-                // a partner that already owns a slot marks it found; the
-                // others are keyed and ordered for creation
-                for (uint32_t q = pass; q; q &= q - 1) {
-                    const int b = i + nl_entry(la, lb, __ffs(q) - 1);
-                    uint32_t hit = 0u;
-                    for (uint32_t left = mask & ((1u << K) - 1u); left; left &= left - 1) {
-                        const int j = __ffs(left) - 1;
-                        if (w.s_b[j * N + i] == b) hit |= 1u << j;
-                    }
-                    if (hit) found_slots |= hit;
-                    else accept_partner(w, b, ca, range_of(w, b), nr);
+            if (!o.search_cells(w, s, nr)) {
+                const int local = (int)w.kbuild[i] - P.cell_base;
+                const int gx = local % P.g_w, gy = local / P.g_w;
+                const int cy0 = max(gy - P.stencil, 0), cy1 = min(gy + P.stencil, P.g_h - 1);
+                const int cx0 = max(gx - P.stencil, 0), cx1 = min(gx + P.stencil, P.g_w - 1);
+                for (int cy = cy0; cy <= cy1; ++cy) {
+                    const int row = P.cell_base + cy * P.g_w;
+                    const int beg = w.cell_start[row + cx0], end = w.cell_start[row + cx1 + 1];
+                    for (int k = beg; k < end; ++k) narrow_test(w, i, w.sorted[k], o, nr);
                 }
             }
+        }
+        if ((listed ? __popc(pass) : nr.cnt) == K) atomicAdd(&w.stats[0], 1ull);
+        changed = !listed || (cm & CM_STALE) != 0u || !cm_unchanged(cm, pass);
+        if (changed && listed) {
+            // the candidate number of each slot's partner, 4 bits a slot (0: not a candidate)
+            uint64_t at = 0u;
+            if (Own::RESIDENT && !(cm & CM_STALE)) {
+                at = o.slot_candidates();
+            } else {
+                for (uint32_t left = mask & SLOT_BITS; left; left &= left - 1) {
+                    const int j = __ffs(left) - 1;
+                    at |= (uint64_t)nl_find(la, lb, o.slot_b(w, j) - i) << (4 * j);
+                }
+            }
+            // delete contacts that were not found (:185-204)
+            uint32_t owned = 0u;  // accepted candidates that own a slot
+            for (uint32_t left = mask & SLOT_BITS; left; left &= left - 1) {
+                const int j = __ffs(left) - 1;
+                const uint32_t hit = pass & ((1u << ((uint32_t)(at >> (4 * j)) & 15u)) & ~1u);
+                owned |= hit;
+                if (hit) continue;
+                const bool bonded_nn = (mask >> (BSHIFT + j)) & 1u;   // bonded >= 0
+                if (!bonded_nn || bonds_model == 0) {
+                    mask &= ~(1u << j);
+                } else if (bonds_model <= 1 && o.slot_bonded(w, j) > 0) {
+                    o.set_tf(w, j, 0.0f);
+                }
+            }
+            // create new contacts in the last empty slot (:207-227), in order
+            // of first shared bucket, then index; one alone needs no order
+            uint32_t fresh = pass & ~owned;
+            const bool ordered = (fresh & (fresh - 1u)) != 0u;
+            if (ordered)
+                for (uint32_t q = fresh; q; q &= q - 1) {
+                    const int k = __ffs(q) - 1, b = i + nl_entry(la, lb, k);
+                    unsigned rank;
+                    shared_bucket(w, ca, o.partner_range(w, b), rank);
+                    top14_insert((rank << 28) | (uint32_t)__ldg(&w.orig[b]), k, nr);
+                }
+            for (int q = 0; fresh; ++q, fresh &= fresh - 1) {
+                const int k = ordered ? nr.idx(q) : __ffs(fresh) - 1;
+                const uint32_t empty = (~mask) & SLOT_BITS;
+                if (empty == 0u) continue;
+                const int j = 31 - __clz(empty);
+                mask |= 1u << j;
+                o.new_slot(w, j, i + nl_entry(la, lb, k));
+                at = (at & ~((uint64_t)15u << (4 * j))) | (uint64_t)k << (4 * j);
+            }
+            // the match word of the slots as they are now
+            if (mask & NL_LIVE) {
+                uint32_t next = CM_STALE;
+                if (bonds_model != 1) {
+                    next = 0u;
+                    for (uint32_t left = mask & SLOT_BITS; left; left &= left - 1) {
+                        const int j = __ffs(left) - 1;
+                        const uint32_t c = (1u << ((uint32_t)(at >> (4 * j)) & 15u)) & ~1u;
+                        next |= c;
+                        if (bonds_model == 0 || !((mask >> (BSHIFT + j)) & 1u)) next |= c << 16;
+                    }
+                }
+                if (next != cm) o.set_match(w, next);
+            }
+            o.set_slot_candidates(at);
+        } else if (changed) {
             const int cnt = nr.cnt;
-            // delete contacts that were not found (:185-204); `matched` marks the
+            // as above with the partners themselves: `matched` marks the
             // accepted partners that already own a slot
             uint32_t matched = 0u;
-            for (uint32_t left = mask & ((1u << K) - 1u); left; left &= left - 1) {
+            for (uint32_t left = mask & SLOT_BITS; left; left &= left - 1) {
                 const int j = __ffs(left) - 1;
-                bool found = (found_slots >> j) & 1u;
-                if (!listed) {
-                    const int sb = w.s_b[j * N + i];
-                    for (int q = 0; q < cnt; ++q) {
-                        const bool hit = nr_ci[q * IB + t] == sb;
-                        found |= hit;
-                        matched |= hit ? (1u << q) : 0u;
-                    }
+                bool found = false;
+                const int sb = o.slot_b(w, j);
+                for (int q = 0; q < cnt; ++q) {
+                    const bool hit = nr.idx(q) == sb;
+                    found |= hit;
+                    matched |= hit ? (1u << q) : 0u;
                 }
                 if (found) continue;
                 const bool bonded_nn = (mask >> (BSHIFT + j)) & 1u;   // bonded >= 0
                 if (!bonded_nn || bonds_model == 0) {
                     mask &= ~(1u << j);
-                } else if (bonds_model <= 1 && w.s_bonded[j * N + i] > 0) {
-                    w.s_tf[j * N + i] = 0.0f;
+                } else if (bonds_model <= 1 && o.slot_bonded(w, j) > 0) {
+                    o.set_tf(w, j, 0.0f);
                 }
             }
-            // create new contacts in the last empty slot (:207-227); a deleted
-            // slot never holds an accepted partner, so `matched` is the
-            // reference's "existing" test
+            // a deleted slot never holds an accepted partner, so `matched` is
+            // the reference's "existing" test
             for (int q = 0; q < cnt; ++q) {
                 if ((matched >> q) & 1u) continue;
-                const uint32_t empty = (~mask) & ((1u << K) - 1u);
+                const uint32_t empty = (~mask) & SLOT_BITS;
                 if (empty == 0u) continue;
                 const int j = 31 - __clz(empty);
                 mask |= 1u << j;
-                w.s_b[j * N + i] = nr_ci[q * IB + t];
-                w.s_tf[j * N + i] = 0.0f;
+                o.new_slot(w, j, nr.idx(q));
             }
-            // the match word of the slots as they are now
-            if (mask & NL_LIVE) {
-                uint32_t next = CM_STALE;
-                if (listed && bonds_model != 1) {
-                    next = 0u;
-                    for (uint32_t left = mask & ((1u << K) - 1u); left; left &= left - 1) {
-                        const int j = __ffs(left) - 1;
-                        const int off = w.s_b[j * N + i] - i;
-                        uint32_t at = 0u;
-                        for (int k = 1; k <= lc; ++k) at |= nl_entry(la, lb, k) == off ? 1u << k : 0u;
-                        next |= at;
-                        if (bonds_model == 0 || !((mask >> (BSHIFT + j)) & 1u)) next |= at << 16;
-                    }
-                }
-                if (next != cm) w.cmask[i] = next;
-            }
+            if ((mask & NL_LIVE) && cm != CM_STALE) o.set_match(w, CM_STALE);
         }
     }
 
     if (PART == 1) {
-        if (mask != before) w.smask[i] = mask;
+        o.set_mask(w, mask, before);
         return;
     }
 
@@ -1483,44 +1675,31 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
     // Per slot, every load is issued before any result is used: the slot
     // fields, then what they index (partner records, bond records), so a
     // slot costs two dependent memory round trips instead of five.
-    const float4 da = (mask & ((1u << K) - 1u)) ? w.dp[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float4 da = (mask & SLOT_BITS) ? o.disp(w) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float nfx = 0.0f, nfy = 0.0f, nm = 0.0f;
     Acc3 acc = {0.0f, 0.0f, 0.0f};
-    for (uint32_t left = mask & ((1u << K) - 1u); left; left &= left - 1) {
+    uint32_t left = mask & SLOT_BITS;
+    if (Own::RESIDENT && changed && left) ahead = fetch(__ffs(left) - 1);
+    while (left) {
         const int j = __ffs(left) - 1;
-        const bool bnn = (mask >> (BSHIFT + j)) & 1u;              // bonded >= 0
-        const int b = w.s_b[j * N + i];
-        const float tf0 = w.s_tf[j * N + i];
-        int bonded = -1;                                           // any negative value acts alike
-        float btf0 = 0.0f, thb0 = 0.0f;
-        if (bnn) {
-            bonded = w.s_bonded[j * N + i];
-            if (bonds_model == 3) {
-                btf0 = w.s_btf[j * N + i];
-                thb0 = w.s_thb[j * N + i];
-            }
-        }
-        const float4 pb = __ldg(&w.pr[b]);
-        const float4 db = __ldg(&w.dp[b]);
-        const uint32_t mb = U.n_mat == 1 ? 0u : __ldg(&w.meta[b]);
-        int st = 0;
-        float blen = 0.0f;
-        float2 str = make_float2(U.p.bond_normal_strength, U.p.bond_shear_strength);
-        if (bnn) {
-            const int bg = P.bond_base + bonded;
-            st = w.b_status[bg];
-            blen = w.b_length[bg];
-            if (U.has_strength) str = w.b_str[bg];
-        }
+        left &= left - 1;
+        const SlotIn in = Own::RESIDENT ? ahead : fetch(j);
+        if (Own::RESIDENT && left) ahead = fetch(__ffs(left) - 1);
+        const int b = in.b, st = in.st;
+        const float tf0 = in.tf, btf0 = in.btf, thb0 = in.thb, blen = in.blen;
+        const float4 pb = in.pb, db = in.db;
+        const uint32_t mb = in.mb;
+        const float2 str = in.str;
+        int bonded = in.bonded;
         if (st < 0) {                                              // :236-239
-            w.s_bonded[j * N + i] = st;
+            o.set_bonded(w, j, st);
             bonded = st;
             mask &= ~(1u << (BSHIFT + j));
         }
-        const float2 kns = __ldg(&w.pair[P.pair_base + (int)meta_mat(m) * U.n_mat + (int)meta_mat(mb)]);
+        const float2 kns = o.stiffness(w, U.n_mat, P.pair_base + (int)meta_mat(m) * U.n_mat + (int)meta_mat(mb));
         float meff = 0.0f;  // effective mass of the pair, for the dashpot (generic form only)
         if (MAY_F64 && U.damp2 > 0.0f) {
-            const float ma = ((w.mats[P.mat_base + meta_mat(m)].density * 3.14159274101257324219f) * pa.z) * pa.z;
+            const float ma = ((o.density(w, P.mat_base + (int)meta_mat(m)) * 3.14159274101257324219f) * pa.z) * pa.z;
             const float mbb = ((w.mats[P.mat_base + meta_mat(mb)].density * 3.14159274101257324219f) * pb.z) * pb.z;
             meff = (ma * mbb) / (ma + mbb);
         }
@@ -1532,7 +1711,7 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
             float tf = tf0;
             f = linear_model<MAY_F64>(U, kns, pa, da, pb, db, pa.z + pb.z, len2f(pa.x - pb.x, pa.y - pb.y), tf, acc,
                                      meff);
-            w.s_tf[j * N + i] = tf;
+            o.set_tf(w, j, tf);
         } else {
             const int bg = P.bond_base + bonded;
             const float sn = str.x, ss = str.y;
@@ -1566,8 +1745,9 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
                     ((Fn / A) - (U.p.moment_contribution_factor * (bend * Rr)) / I < -sn ||
                      abtf / A > ss)) {
                     const int code = -10 + sign_i32(nd);
-                    record_break(w, P, s, *w.step, bg, code, i, b);
-                    w.s_bonded[j * N + i] = code;
+                    record_break(w, P, s, o.step(w), bg, code, i, b);
+                    o.broke();
+                    o.set_bonded(w, j, code);
                     mask &= ~(1u << (BSHIFT + j));
                     Fn = 0.0f;
                     btf = 0.0f;
@@ -1575,14 +1755,14 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
                     Fy = 0.0f;
                     M = 0.0f;
                 }
-                w.s_btf[j * N + i] = btf;
-                w.s_thb[j * N + i] = thb;
+                o.set_btf(w, j, btf);
+                o.set_thb(w, j, thb);
                 acc.d0 = acc.d0 + (-Fn);
                 acc.d1 = acc.d1 + btf;
                 acc.d2 = acc.d2 + M;
                 float tf = tf0;
                 const F3 lm = linear_model<MAY_F64>(U, kns, pa, da, pb, db, blen, L, tf, acc, meff);
-                w.s_tf[j * N + i] = tf;
+                o.set_tf(w, j, tf);
                 f.x = Fx + lm.x;
                 f.y = Fy + lm.y;
                 f.z = M + lm.z;
@@ -1596,15 +1776,16 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
                 fy = fy + sf * (vy / L);
                 if (U.p.bonds_tear == 1 && sf >= sn) {
                     const int code = -10 + sign_i32(disp);
-                    record_break(w, P, s, *w.step, bg, code, i, b);
-                    w.s_bonded[j * N + i] = code;
+                    record_break(w, P, s, o.step(w), bg, code, i, b);
+                    o.broke();
+                    o.set_bonded(w, j, code);
                     mask &= ~(1u << (BSHIFT + j));
                     fx = 0.0f;
                     fy = 0.0f;
                 }
                 float tf = tf0;
                 const F3 lm = linear_model<MAY_F64>(U, kns, pa, da, pb, db, blen, L, tf, acc, meff);
-                w.s_tf[j * N + i] = tf;
+                o.set_tf(w, j, tf);
                 f.x = lm.x + fx;
                 f.y = lm.y + fy;
                 f.z = lm.z + 0.0f;
@@ -1630,16 +1811,17 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
                 const float atf = tf < 0.0f ? -tf : tf;
                 if (U.p.bonds_tear == 1 && (Fn < -sn || atf > ss)) {
                     const int code = -10 + sign_i32(nd);
-                    record_break(w, P, s, *w.step, bg, code, i, b);
-                    w.s_bonded[j * N + i] = code;
+                    record_break(w, P, s, o.step(w), bg, code, i, b);
+                    o.broke();
+                    o.set_bonded(w, j, code);
                     mask &= ~(1u << (BSHIFT + j));
                     Fn = 0.0f;
-                    w.s_btf[j * N + i] = 0.0f;
+                    o.set_btf(w, j, 0.0f);
                     Fx = 0.0f;
                     Fy = 0.0f;
                     M = 0.0f;
                 }
-                w.s_tf[j * N + i] = tf;
+                o.set_tf(w, j, tf);
                 acc.d0 = -Fn;
                 acc.d1 = tf;
                 acc.d2 = M;
@@ -1654,12 +1836,11 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
     }
 
     // store_forces (:434-478)
-    const Mat MA = w.mats[P.mat_base + meta_mat(m)];
     const float r = pa.z;
-    const float mass = ((MA.density * 3.14159274101257324219f) * r) * r;
+    const float mass = ((o.density(w, P.mat_base + (int)meta_mat(m)) * 3.14159274101257324219f) * r) * r;
     const float rot_inertia = ((0.5f * mass) * r) * r;
     float4 fe = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (m & M_FEXT) fe = w.fx[i];
+    if (m & M_FEXT) fe = o.external(w);
     float fxs = nfx + fe.x;
     float fys = nfy + fe.y;
     float moment = nm + fe.z;
@@ -1682,23 +1863,24 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
     }
     const float ax = fxs / mass, ay = fys / mass;
     const float al = moment / rot_inertia;
-    const long long rem = FUSE ? w.remaining[s] : 0;
+    const long long rem = FUSE ? o.left(w, s) : 0;
     const bool steps_on = FUSE && rem > 1;  // this scene's next step is in this call
     if (!steps_on) w.ac[i] = make_float4(ax, ay, al, 0.0f);
-    float4 v = w.vw[i];
+    float4 v = o.vel(w);
     const float dT = U.p.dT;
     if (m & M_KICK_X) v.x = v.x + (0.5f * ax) * dT;
     if (m & M_KICK_Y) v.y = v.y + (0.5f * ay) * dT;
     if (m & M_KICK_R) v.z = v.z + (0.5f * al) * dT;
-    if (!FUSE) {
-        w.vw[i] = v;
-    } else if (steps_on) {
-        lom_core(w, P, U, i, m, pa, v, make_float4(ax, ay, al, 0.0f), w.pbuild[i], false,
-                 make_float4(0.0f, 0.0f, 0.0f, 0.0f), lom_final || rem == 2, w.pr_n, w.dp_n);
-    } else {
-        w.vw[i] = v;
-        w.pr_n[i] = pa;
-        w.dp_n[i] = w.dp[i];
+    o.record(w, pa, v.w, acc.d0, acc.d1, acc.d2);
+    if (!steps_on) o.set_vel(w, v);
+    if (steps_on) {
+        float4 p = pa, d, d4;
+        bool moved;
+        lom_core(P, U, m, p, v, make_float4(ax, ay, al, 0.0f), o.rebuilt_at(w), false,
+                 make_float4(0.0f, 0.0f, 0.0f, 0.0f), d, d4, moved);
+        o.advance(w, p, v, d, d4, moved, lom_final || rem == 2);
+    } else if (FUSE) {
+        o.stay(w);
     }
     // data[0..2]; a particle without contacts writes +0 every step, which the
     // slot word's DF_ZERO bit (set while the stored value is all +0) lets it skip
@@ -1707,13 +1889,12 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Narr
         if (!(zero && (mask & DF_ZERO))) w.dF[i] = make_float4(acc.d0, acc.d1, acc.d2, 0.0f);
         mask = zero ? (mask | DF_ZERO) : (mask & ~DF_ZERO);
     }
-    if (mask != before) {
-        w.smask[i] = mask;
-        // a bond broke: its slot is a plain contact from now on
-        if (((mask ^ before) & ~mask & BONDED_BITS) != 0u) w.cmask[i] = CM_STALE;
-    }
+    o.set_mask(w, mask, before);
+    // a bond broke: its slot is a plain contact from now on
+    if (((mask ^ before) & ~mask & BONDED_BITS) != 0u) o.set_match(w, CM_STALE);
 }
 
+#ifndef DEM_STEP_DEVICE_CODE
 // End of step, run by the last warp of k_interact or by k_end_step's block: breaks of this step
 // become visible (status = min code), the positions-set flags clear
 // (2D_Simulation.wgsl:258-261), the step counter advances, and each scene's
@@ -1756,6 +1937,9 @@ __device__ __forceinline__ void interact_tail(const DevWorld &w, bool fused, int
         cudaGraphSetConditional(cond, *(volatile int32_t *)w.rebuild != 0 ? 1u : 0u);
 }
 
+__shared__ uint32_t nr_ck[K * IB];  // Narrow's arrays of k_interact and k_narrow
+__shared__ int nr_ci[K * IB];
+
 // Minimum blocks per SM: measured on GB300 (c3 mix, c2 scene).  Occupancy
 // outweighs the few spilled words down to 40 registers for k_interact (12
 // blocks: 7 % faster than 8) and 56 for k_forces (9 blocks).
@@ -1764,28 +1948,34 @@ __device__ __forceinline__ void interact_tail(const DevWorld &w, bool fused, int
 template <bool FUSE, int FORM, int PS>
 __global__ void __launch_bounds__(IB, 12) k_interact(DevWorld w, int in_graph, cudaGraphConditionalHandle cond,
                                                     int lom_final, const __grid_constant__ ScenePar pv) {
-    Narrow nr;
-    nr.cnt = 0;
+    Narrow<IB> nr{nr_ck + threadIdx.x, nr_ci + threadIdx.x};
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < w.N && chunk_live(w, i)) interact_particle<0, FUSE, FORM, PS>(w, i, nr, lom_final != 0, pv);
+    if (i < w.N && chunk_live(w, i)) {
+        HbmOwn<0, FUSE> o(w, i);
+        interact_particle<0, FUSE, FORM, PS>(w, i, o, nr, lom_final != 0, pv);
+    }
     interact_tail(w, FUSE, in_graph, cond);
 }
 
 template <int FORM, int PS>
 __global__ void __launch_bounds__(IB, 12) k_narrow(DevWorld w, const __grid_constant__ ScenePar pv) {
-    Narrow nr;
-    nr.cnt = 0;
+    Narrow<IB> nr{nr_ck + threadIdx.x, nr_ci + threadIdx.x};
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < w.N && chunk_live(w, i)) interact_particle<1, false, FORM, PS>(w, i, nr, false, pv);
+    if (i < w.N && chunk_live(w, i)) {
+        HbmOwn<1, false> o(w, i);
+        interact_particle<1, false, FORM, PS>(w, i, o, nr, false, pv);
+    }
 }
 
 template <bool FUSE, int FORM, int PS>
 __global__ void __launch_bounds__(IB, 9) k_forces(DevWorld w, int in_graph, cudaGraphConditionalHandle cond,
                                                   int lom_final, const __grid_constant__ ScenePar pv) {
-    Narrow nr;
-    nr.cnt = 0;
+    Narrow<IB> nr{nullptr, nullptr};
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < w.N && chunk_live(w, i)) interact_particle<2, FUSE, FORM, PS>(w, i, nr, lom_final != 0, pv);
+    if (i < w.N && chunk_live(w, i)) {
+        HbmOwn<2, FUSE> o(w, i);
+        interact_particle<2, FUSE, FORM, PS>(w, i, o, nr, lom_final != 0, pv);
+    }
     interact_tail(w, FUSE, in_graph, cond);
 }
 
@@ -2409,5 +2599,7 @@ void launch_set_properties(const DevWorld &w, int scene, const int32_t *d_sel, i
     if (w.N == 0) return;
     k_set_properties<<<(w.N + block - 1) / block, block, 0, st>>>(w, scene, d_sel, d_sel_out, d_props);
 }
+
+#endif  // DEM_STEP_DEVICE_CODE
 
 }  // namespace demgb

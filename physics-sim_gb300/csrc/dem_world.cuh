@@ -36,7 +36,8 @@ constexpr int K = DEM_MAX_CONTACTS;
 constexpr int BSHIFT = 16;  // first bonded-field bit of the slot word
 constexpr uint32_t DF_ZERO = 1u << 31;  // slot-word bit: dF holds +0, +0, +0
 constexpr uint32_t NL_LIVE = 1u << 14;  // slot-word bit: the candidate list is not empty
-constexpr uint32_t BONDED_BITS = ((1u << K) - 1u) << BSHIFT;
+constexpr uint32_t SLOT_BITS = (1u << K) - 1u;            // slot-word bits: occupied slots
+constexpr uint32_t BONDED_BITS = SLOT_BITS << BSHIFT;     // and: slot's bonded field >= 0
 constexpr uint32_t CM_STALE = 1u;       // match word: nothing is known (see DevWorld::cmask)
 
 // meta word: fixity predicates, external-force flag, material, scene
@@ -118,6 +119,26 @@ struct Pending {
     int32_t bond, code;
 };
 
+// A run of steps in one kernel (dem_steps.cu): what is left of it, its
+// barrier, and the particles whose datum it records after every step.
+struct StepRun {
+    int32_t todo, done;      // steps left and taken of the call
+    int32_t lom_done;        // 1: the next step's LOM pass has run
+    uint32_t arrive[3];      // barrier counters, used in turn
+    uint32_t gen;            // the launch's last barrier whose breaks have been applied
+    uint32_t fail;           // a wait gave up: no run starts any more
+    uint32_t links;          // rebuilds by cell chains so far (a chain's number is never 0)
+    int32_t linked;          // 1: the lists come from such a rebuild, and cell_start and sorted are of an earlier one
+    int32_t rec_scene, rec_base, rec_per;  // recorded scene, its first particle, floats a step
+    const int32_t *rec_rows; // [particles of the scene] row of each recorded one, -1 the others; null: none
+    float *rec_out;
+};
+// before every launch of the kernel
+__device__ __forceinline__ void clear_run_barrier(StepRun &R) {
+    R.arrive[0] = R.arrive[1] = R.arrive[2] = 0u;
+    R.gen = 0u;
+}
+
 struct DevWorld {
     int32_t N, C, B, S, M, MP;
     float4 *pr, *vw, *ac, *dp, *fx, *d4, *dF;
@@ -177,6 +198,9 @@ struct DevWorld {
     int32_t *big_acc;           // [slots][16]: accepted partners of a large particle, [15] = count
     int32_t *big_scene;         // [slots] scene of each big-partner record, -1 unused
     int32_t n_big_slots;
+    StepRun *run;
+    unsigned long long *cell_head;  // [C] cell chains (worlds of resident runs): rebuild number << 32 | last particle
+    int32_t *cell_next;             // [N] the particle put in before it, -1: none
     int32_t *det;               // [S] narrow phase runs in the current step
     const uint8_t *live;        // [ceil(N/128)] 0: every particle of the 128-particle chunk is free
                                 // (served worlds: the step kernels skip it); null: all chunks live
@@ -236,6 +260,24 @@ int launch_list_build(const DevWorld &w, int block, cudaStream_t st, const int32
 constexpr int PS_SCENE = 0, PS_SHARED = 1, PS_ONE = 2;
 int launch_interact(const DevWorld &w, int block, cudaStream_t st, bool bigs, bool fuse, bool lom_final,
                     bool in_graph, cudaGraphConditionalHandle cond, int form, const ScenePar *pv, int ps);
+
+// Runs of steps in one kernel (dem_steps.cu), for worlds of at most one
+// particle a thread, 512 threads an SM, without large particles.
+// steps_block: the block size for n particles, 0 when the device or the size
+// does not allow it.  launch_run_begin: the next run takes `todo` steps.
+// launch_steps: captured in a graph's while node; the kernel sets `rebuild`
+// when the lists must be rebuilt before it goes on, and `more` until every
+// step is done.
+struct RunRecord {
+    const int32_t *rows = nullptr;
+    int scene = 0, base = 0, per = 0;
+    float *out = nullptr;
+};
+int device_sms();  // SMs of the current device
+int steps_block(int n);
+void launch_run_begin(const DevWorld &w, int todo, const RunRecord &rec, cudaStream_t st);
+cudaError_t launch_steps(const DevWorld &w, int block, cudaStream_t st, cudaGraphConditionalHandle more,
+                         cudaGraphConditionalHandle rebuild, int form, const ScenePar *pv, int ps);
 
 // The fields of a scene's parameters that the Simulation kernels read from
 // the launch under PS_SHARED (the settings and model constants), the others

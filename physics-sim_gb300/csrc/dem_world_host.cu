@@ -82,6 +82,7 @@ World::~World() {
     if (d_copies) cudaFree(d_copies);
     for (auto e : xfer_ev) cudaEventDestroy(e);
     if (side) cudaStreamDestroy(side);
+    if (side2) cudaStreamDestroy(side2);
 }
 
 // staging area for one scene of n particles in the reference layouts:
@@ -514,7 +515,7 @@ int World::alloc(int N, int C, int B, int S, int M, int MP, int TB, uint32_t ev_
     // default: every 3rd rebuild in a single-scene world (a dense scene's
     // warps gain from fresh grouping by contact count), every 8th in a
     // batch or server (many sparse scenes: the reorder's bytes dominate)
-    w.reorder_every = reorder_every > 0 ? reorder_every : (S == 1 ? 3 : 8);
+    w.reorder_every = reorder_every > 0 ? reorder_every : (S == 1 ? 3 : 8);  // see refresh_graphs
     w.tickets = dalloc<uint32_t>(owned, 2, ok);
     w.fix_ref = dalloc<int32_t>(owned, 6 * (size_t)N, ok);
     w.force_ref = dalloc<float>(owned, 6 * (size_t)N, ok);
@@ -523,6 +524,10 @@ int World::alloc(int N, int C, int B, int S, int M, int MP, int TB, uint32_t ev_
     w.n_big_slots = TB;
     w.big_acc = dalloc<int32_t>(owned, 16 * (size_t)std::max(TB, 1), ok);
     w.big_scene = dalloc<int32_t>(owned, std::max(TB, 1), ok);
+    w.run = dalloc<StepRun>(owned, 1, ok);
+    run_block = steps_block(N);
+    w.cell_head = dalloc<unsigned long long>(owned, run_block ? (size_t)C : 1, ok);
+    w.cell_next = dalloc<int32_t>(owned, run_block ? (size_t)N : 1, ok);
     w.det = dalloc<int32_t>(owned, S, ok);
     w.act = dalloc<int32_t>(owned, S, ok);
     w.remaining = dalloc<long long>(owned, S, ok);
@@ -539,6 +544,8 @@ int World::alloc(int N, int C, int B, int S, int M, int MP, int TB, uint32_t ev_
     CK(cudaMemsetAsync(w.tickets, 0, 2 * sizeof(uint32_t), stream));
     CK(cudaMemsetAsync(w.nl, 0, sizeof(int4) * 2 * (size_t)(N > 0 ? N : 1), stream));
     CK(cudaMemsetAsync(w.err, 0, sizeof(int32_t), stream));
+    CK(cudaMemsetAsync(w.run, 0, sizeof(StepRun), stream));
+    if (run_block) CK(cudaMemsetAsync(w.cell_head, 0, 8 * (size_t)C, stream));
     {
         static const int32_t one = 1;  // the first rebuild reorders
         CK(cudaMemcpyAsync(w.reorder, &one, 4, cudaMemcpyHostToDevice, stream));
@@ -1656,7 +1663,8 @@ void World::drop_graph() {
     for (int p = 0; p < 2; ++p) {
         if (graph[p]) cudaGraphExecDestroy(graph[p]);
         if (graph1[p]) cudaGraphExecDestroy(graph1[p]);
-        graph[p] = graph1[p] = nullptr;
+        if (graph_run[p]) cudaGraphExecDestroy(graph_run[p]);
+        graph[p] = graph1[p] = graph_run[p] = nullptr;
         graph_R[p] = 0;
     }
 }
@@ -1771,6 +1779,85 @@ int World::capture_graph(int R, cudaGraphExec_t *out, int *kernels_out) {
     return DEM_OK;
 }
 
+// The graph of a run in a small world: while steps are left, k_steps, then
+// the rebuild if it stopped for one.  The run's length is a device word
+// (launch_run_begin), so one graph serves every call.
+int World::capture_run(cudaGraphExec_t *out) {
+    if (!side) CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    if (!side2) CK(cudaStreamCreateWithFlags(&side2, cudaStreamNonBlocking));
+    cudaGraph_t g = nullptr;
+    CK(cudaGraphCreate(&g, 0));
+    cudaGraphConditionalHandle more{}, due{};
+    const auto conditional = [](cudaGraph_t in, const cudaGraphNode_t *deps, size_t n, cudaGraphConditionalHandle h,
+                                cudaGraphConditionalNodeType type, cudaGraphNode_t *node, cudaGraph_t *body) {
+        cudaGraphNodeParams np = {cudaGraphNodeTypeConditional};
+        np.type = cudaGraphNodeTypeConditional;
+        np.conditional.handle = h;
+        np.conditional.type = type;
+        np.conditional.size = 1;
+        const cudaError_t e = cudaGraphAddNode(node, in, deps, nullptr, n, &np);
+        if (e == cudaSuccess) *body = np.conditional.phGraph_out[0];
+        return e;
+    };
+    cudaGraphNode_t loop, branch;
+    cudaGraph_t body = nullptr, lists = nullptr;
+    cudaError_t e = cudaGraphConditionalHandleCreate(&more, g, 1, cudaGraphCondAssignDefault);
+    if (e == cudaSuccess) e = conditional(g, nullptr, 0, more, cudaGraphCondTypeWhile, &loop, &body);
+    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&due, body, 0, cudaGraphCondAssignDefault);
+    if (e == cudaSuccess)
+        e = cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+        cudaGraph_t done = nullptr;
+        e = launch_steps(d, run_block, side, more, due, kernel_form, &par_pv, par_ps);
+        const cudaGraphNode_t *deps = nullptr;
+        size_t ndeps = 0;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (e == cudaSuccess) e = cudaStreamGetCaptureInfo(side, &cs, nullptr, nullptr, &deps, nullptr, &ndeps);
+        if (e == cudaSuccess && cs != cudaStreamCaptureStatusActive) e = cudaErrorStreamCaptureInvalidated;
+        if (e == cudaSuccess) e = conditional(body, deps, ndeps, due, cudaGraphCondTypeIf, &branch, &lists);
+        if (e == cudaSuccess)
+            e = cudaStreamBeginCaptureToGraph(side2, lists, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+        if (e == cudaSuccess) {
+            enqueue_rebuild(side2, d.rebuild, false);
+            e = cudaGetLastError();
+            const cudaError_t e2 = cudaStreamEndCapture(side2, &done);
+            if (e == cudaSuccess) e = e2;
+        }
+        if (e == cudaSuccess)
+            e = cudaStreamUpdateCaptureDependencies(side, &branch, nullptr, 1, cudaStreamSetCaptureDependencies);
+        const cudaError_t e3 = cudaStreamEndCapture(side, &done);
+        if (e == cudaSuccess) e = e3;
+    }
+    cudaGraphExec_t ex = nullptr;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) return fail(DEM_E_CUDA, std::string("graph of a run: ") + cudaGetErrorString(e));
+    *out = ex;
+    return DEM_OK;
+}
+
+// Whether a step call is one run of k_steps.  Every world whose particles
+// fit one a thread takes it (a launch a step -> a run, microseconds a step:
+// 128 bonded particles 19.4 -> 4.9, 4,096 falling 13.8 -> 3.7, 16,384 bonded
+// 18.2 -> 6.9, a 30,011-particle bed with F64 distances 35.9 -> 15, its FP32
+// form of 70,000 33.6 -> 13.7); k_big_narrow is a launch of its own.
+bool World::runs_resident() const { return use_graphs && !timing && !has_bigs && run_block > 0; }
+
+// one run of n_steps, recording the datum of the particles in rec.rows
+int World::run_steps(int n_steps, const RunRecord &rec) {
+    const int p = parity;
+    if (!graph_run[p]) {
+        const int rc = capture_run(&graph_run[p]);
+        if (rc) return rc;
+    }
+    launch_run_begin(d, n_steps, rec, stream);
+    CK(cudaGetLastError());
+    CK(cudaGraphLaunch(graph_run[p], stream));
+    launches += 2;
+    host_step += n_steps;
+    return DEM_OK;
+}
+
 // the scene parameters' source for the Simulation launches of a step() call:
 // the host records equal the device's whenever a call steps
 void World::update_param_source() {
@@ -1829,17 +1916,39 @@ void World::update_split() {
     drop_graph();
 }
 
-int World::step(int n_steps) {
-    if (n_steps < 0) return fail(DEM_E_INVALID, "n_steps < 0");
+// what the captured graphs depend on, brought up to date before a call steps
+int World::refresh_graphs() {
     update_param_source();
     update_split();
+    const bool resident = runs_resident();
+    // the records of a world that runs resident sit in L2 wherever they are:
+    // its rebuilds stay within the run, all but one in 32
+    const int every = reorder_every > 0 ? reorder_every : resident ? 32 : (sh.size() == 1 ? 3 : 8);
+    if (every != d.reorder_every) {
+        d.reorder_every = every;
+        drop_graph();
+    }
+    if (was_resident && !resident) {
+        // the cell table may be of an earlier rebuild than the lists
+        const int rc = force_rebuild(false);
+        if (rc) return rc;
+    }
+    was_resident = resident;
+    if (par_ps != graph_ps || std::memcmp(&par_pv, &graph_par, sizeof(ScenePar)) != 0) {
+        drop_graph();
+        graph_ps = par_ps;
+        std::memcpy(&graph_par, &par_pv, sizeof(ScenePar));
+    }
+    return DEM_OK;
+}
+
+int World::step(int n_steps) {
+    if (n_steps < 0) return fail(DEM_E_INVALID, "n_steps < 0");
+    const int rc = refresh_graphs();
+    if (rc) return rc;
+    if (n_steps > 0 && runs_resident()) return run_steps(n_steps, RunRecord{});
     int k = 0;
     if (use_graphs && !timing && n_steps > 0) {
-        if (par_ps != graph_ps || std::memcmp(&par_pv, &graph_par, sizeof(ScenePar)) != 0) {
-            drop_graph();
-            graph_ps = par_ps;
-            std::memcpy(&graph_par, &par_pv, sizeof(ScenePar));
-        }
         while (n_steps - k >= graph_steps) {
             const int p = parity;
             if (!graph[p] || graph_R[p] != graph_steps) {
@@ -1878,6 +1987,7 @@ int World::sync() {
     CK(cudaStreamSynchronize(stream));
     int32_t e = 0;
     CK(cudaMemcpy(&e, d.err, 4, cudaMemcpyDeviceToHost));
+    if (e & 8) return fail(DEM_E_TIMEOUT, "a wait between the blocks of a step kernel gave up");
     if (e) return fail(DEM_E_STATE, "device error flags set: " + std::to_string(e));
     return DEM_OK;
 }
@@ -2249,17 +2359,31 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
     }
     const long long per = 10LL * k;  // floats per recorded step
     const int chunk = (int)std::max<long long>(1, std::min<long long>(n_steps, (1LL << 24) / per));
+    // a resident run records inside its kernel, which looks up each particle's
+    // row; else a gather after every step takes the list of recorded particles
+    const bool resident = runs_resident();
+    std::vector<int32_t> row_of;
+    if (resident) {
+        row_of.assign((size_t)h.n, -1);
+        for (int t = 0; t < k; ++t) row_of[idx[t]] = t;
+        idx = row_of;
+    }
     void *dbuf = nullptr;
-    CK(cudaMalloc(&dbuf, sizeof(int32_t) * (size_t)k + sizeof(float) * (size_t)(per * chunk)));
+    CK(cudaMalloc(&dbuf, sizeof(int32_t) * idx.size() + sizeof(float) * (size_t)(per * chunk)));
     int32_t *d_idx = static_cast<int32_t *>(dbuf);
-    float *d_rows = reinterpret_cast<float *>(d_idx + k);
+    const int32_t *d_sel = resident ? d_idx : nullptr;
+    float *d_rows = reinterpret_cast<float *>(d_idx + idx.size());
     std::vector<float> f((size_t)(per * chunk));
     int rc = DEM_OK;
-    cudaError_t e = cudaMemcpyAsync(d_idx, idx.data(), sizeof(int32_t) * k, cudaMemcpyHostToDevice, stream);
+    cudaError_t e = cudaMemcpyAsync(d_idx, idx.data(), sizeof(int32_t) * idx.size(), cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) rc = fail(DEM_E_CUDA, std::string("record: ") + cudaGetErrorString(e));
     for (int s0 = 0; rc == DEM_OK && s0 < n_steps; s0 += chunk) {
         const int m = std::min(chunk, n_steps - s0);
-        for (int j = 0; j < m && rc == DEM_OK; ++j) {
+        if (d_sel) {
+            rc = refresh_graphs();
+            if (rc == DEM_OK) rc = run_steps(m, RunRecord{d_sel, s, h.particle_base, (int)per, d_rows});
+        }
+        for (int j = 0; j < m && rc == DEM_OK && !d_sel; ++j) {
             rc = step(1);
             if (rc == DEM_OK) launch_gather_datum(d, h.particle_base, d_idx, k, d_rows + per * j, stream);
         }

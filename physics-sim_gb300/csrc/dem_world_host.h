@@ -108,7 +108,7 @@ class World {
 
     std::string err;
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;   // captures the rebuild body of a conditional node
+    cudaStream_t side = nullptr, side2 = nullptr;  // capture the bodies of conditional nodes
     int device = 0;
     int block = 256;
     int graph_steps = 35;          // steps per captured CUDA graph
@@ -158,6 +158,13 @@ class World {
     void enqueue_plain_step(bool first, bool last, bool next_last);
     void enqueue_rebuild(cudaStream_t st, const int32_t *gate, bool every_step);
     int capture_graph(int R, cudaGraphExec_t *out, int *kernels);
+    int run_block = 0;             // block size of a resident run (steps_block), 0: none
+    cudaGraphExec_t graph_run[2] = {nullptr, nullptr};  // a run of steps, per buffer parity
+    int capture_run(cudaGraphExec_t *out);
+    bool runs_resident() const;
+    int run_steps(int n_steps, const RunRecord &rec);
+    int refresh_graphs();
+    bool was_resident = false;
     void drop_graph();
     bool dense_cells() const;
     DevWorld spare{};
