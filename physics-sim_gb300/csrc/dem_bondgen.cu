@@ -27,9 +27,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "dem.h"
@@ -114,19 +116,15 @@ __global__ void k_bg_select(const float2 *__restrict__ pos, const float *__restr
     count[i] = nb;
 }
 
-// bond records (status) and the j side's incoming count
+// the two sides of every bond and the j side's incoming count
 __global__ void k_bg_write(int n, int max_bonds, const int32_t *__restrict__ sel,
                            const int32_t *__restrict__ count, const int32_t *__restrict__ base,
-                           int32_t *__restrict__ bonds, int32_t *__restrict__ bond_i, int32_t *__restrict__ bond_j,
-                           int32_t *in_count) {
+                           int32_t *__restrict__ bond_i, int32_t *__restrict__ bond_j, int32_t *in_count) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     for (int q = 0; q < count[i]; ++q) {
         const int b = base[i] + q;
         const int j = sel[(size_t)i * max_bonds + q];
-        bonds[3 * (size_t)b] = 1;
-        bonds[3 * (size_t)b + 1] = 0;  // angle and length: filled on the host
-        bonds[3 * (size_t)b + 2] = 0;
         bond_i[b] = i;
         bond_j[b] = j;
         atomicAdd(&in_count[j], 1);
@@ -145,50 +143,111 @@ struct BgBonds {
     }
 };
 
-// contact slots: bonds where p is the j side (ascending number), then p's own
-__global__ void k_bg_slots(int n, int max_bonds, const int32_t *__restrict__ count, const int32_t *__restrict__ base,
-                           const int32_t *__restrict__ sel, const int32_t *__restrict__ in_start,
-                           const int32_t *__restrict__ in_list, const int32_t *__restrict__ bond_i,
-                           int32_t *__restrict__ contacts) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const int beg = in_start[p], end = in_start[p + 1];
-    int32_t *c = contacts + (size_t)p * K * 6;
-    int s = 0;
-    for (int a = beg; a < end && s < K; ++a, ++s) {
-        const int b = in_list[a];
-        c[6 * s] = p;
-        c[6 * s + 1] = bond_i[b];
-        c[6 * s + 2] = 0;
-        c[6 * s + 3] = 0;
-        c[6 * s + 4] = 0;
-        c[6 * s + 5] = b;
+// contact slots: bonds where p is the j side (ascending number), then p's own.
+// A block builds its particles' records in shared memory and writes them out
+// as one run (a record is 84 words: each thread storing its own touches a
+// sector per word).
+constexpr int BG_SLOTS = 64, BG_REC = 6 * K;
+__global__ void __launch_bounds__(BG_SLOTS) k_bg_slots(int n, int max_bonds, const int32_t *__restrict__ count,
+                                                       const int32_t *__restrict__ base,
+                                                       const int32_t *__restrict__ sel,
+                                                       const int32_t *__restrict__ in_start,
+                                                       const int32_t *__restrict__ in_list,
+                                                       const int32_t *__restrict__ bond_i,
+                                                       int32_t *__restrict__ contacts) {
+    __shared__ int32_t rec[BG_SLOTS * (BG_REC + 1)];  // a word of padding: no two lanes in a bank
+    const int p0 = blockIdx.x * BG_SLOTS, p = p0 + threadIdx.x;
+    if (p < n) {
+        const int beg = in_start[p], end = in_start[p + 1];
+        int32_t *c = rec + threadIdx.x * (BG_REC + 1);
+        int s = 0;
+        const auto put = [&](int partner, int b) {
+            c[6 * s] = p;
+            c[6 * s + 1] = partner;
+            c[6 * s + 2] = 0;
+            c[6 * s + 3] = 0;
+            c[6 * s + 4] = 0;
+            c[6 * s + 5] = b;
+            ++s;
+        };
+        for (int a = beg; a < end && s < K; ++a) put(bond_i[in_list[a]], in_list[a]);
+        for (int q = 0; q < count[p] && s < K; ++q) put(sel[(size_t)p * max_bonds + q], base[p] + q);
+        for (int f = 6 * s; f < BG_REC; ++f) c[f] = -1;
     }
-    for (int q = 0; q < count[p] && s < K; ++q, ++s) {
-        c[6 * s] = p;
-        c[6 * s + 1] = sel[(size_t)p * max_bonds + q];
-        c[6 * s + 2] = 0;
-        c[6 * s + 3] = 0;
-        c[6 * s + 4] = 0;
-        c[6 * s + 5] = base[p] + q;
-    }
-    for (; s < K; ++s)
-        for (int f = 0; f < 6; ++f) c[6 * s + f] = -1;
+    __syncthreads();
+    const int words = (n - p0 < BG_SLOTS ? n - p0 : BG_SLOTS) * BG_REC;
+    int32_t *out = contacts + (size_t)p0 * BG_REC;
+    for (int f = threadIdx.x; f < words; f += BG_SLOTS) out[f] = rec[f / BG_REC * (BG_REC + 1) + f % BG_REC];
 }
 
-struct DevBuf {
-    std::vector<void *> ptrs;
-    ~DevBuf() {
-        for (void *p : ptrs) cudaFree(p);
-    }
+// Arrays carved from one device allocation: `take` is called once without a
+// base, to add up the size, and once with it.
+struct Carve {
+    char *base = nullptr;
+    size_t bytes = 0;
     template <class T>
-    T *get(size_t count) {
-        void *p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) return nullptr;
-        ptrs.push_back(p);
-        return static_cast<T *>(p);
+    T *take(size_t count) {
+        T *p = base ? reinterpret_cast<T *>(base + bytes) : nullptr;
+        bytes += (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255;
+        return p;
     }
 };
+struct DevBlock {
+    void *p = nullptr;
+    ~DevBlock() {
+        if (p) cudaFree(p);
+    }
+    template <class Layout>
+    bool carve(Layout layout) {
+        Carve c;
+        layout(c);
+        if (cudaMalloc(&p, c.bytes) != cudaSuccess) {
+            p = nullptr;
+            cudaGetLastError();
+            return false;
+        }
+        c = Carve{static_cast<char *>(p), 0};
+        layout(c);
+        return true;
+    }
+};
+
+// Length and angle of every bond with the host's powf and atan2f, ~25 ns a
+// bond, in chunks taken by up to 8 threads: the caller works too, so a thread
+// that cannot be started costs time only.  200,003 particles, 238,396 bonds:
+// a call 9.6 -> 2.8 ms, with the arrays in two device allocations instead of
+// twenty (0.7 ms) and the contact records' copy behind this.
+// length = (dx*dx + dy*dy)^0.5, angle = atan2(dx / |d|, dy / |d|) (state.rs:309-313)
+void bond_records(const float *pos, const int32_t *bi, const int32_t *bj, int32_t total, int32_t *bonds) {
+    constexpr int32_t CHUNK = 4096;
+    alignas(256) std::atomic<int32_t> next{0};
+    const int32_t chunks = (int32_t)(((long long)total + CHUNK - 1) / CHUNK);
+    // captured by value: the caller writes the lines of its stack as it works,
+    // and a thread that read its arguments there would wait for them (x 10)
+    const auto work = [=, &next]() {
+        for (int32_t c; (c = next.fetch_add(1)) < chunks;) {
+            const int32_t end = (int32_t)std::min<long long>(total, ((long long)c + 1) * CHUNK);
+            for (int32_t b = c * CHUNK; b < end; ++b) {
+                const size_t i = (size_t)bi[b], j = (size_t)bj[b];
+                const float dx = pos[2 * j] - pos[2 * i], dy = pos[2 * j + 1] - pos[2 * i + 1];
+                const float mag = std::pow(dx * dx + dy * dy, 0.5f);
+                const float ang = std::atan2(dx / mag, dy / mag);
+                bonds[3 * (size_t)b] = 1;
+                std::memcpy(&bonds[3 * (size_t)b + 1], &ang, 4);
+                std::memcpy(&bonds[3 * (size_t)b + 2], &mag, 4);
+            }
+        }
+    };
+    const int32_t helpers = std::min<int32_t>({chunks - 1, 7, (int32_t)std::thread::hardware_concurrency() - 1});
+    std::vector<std::thread> pool;
+    try {
+        pool.reserve((size_t)std::max(helpers, 0));
+        for (int32_t t = 0; t < helpers; ++t) pool.emplace_back(work);
+    } catch (...) {
+    }
+    work();
+    for (auto &t : pool) t.join();
+}
 
 }  // namespace
 
@@ -239,16 +298,26 @@ int dem_generate_bonds(const float *pos, const float *radii, int32_t n, int32_t 
         return bfail(DEM_E_CUDA, "stream creation failed");
     int rc = DEM_OK;
     {
-        DevBuf db;
-        float2 *d_pos = db.get<float2>(n);
-        float *d_r = db.get<float>(n);
-        int32_t *d_keys = db.get<int32_t>(n), *d_cnt = db.get<int32_t>(cells), *d_start = db.get<int32_t>(cells + 1);
-        int32_t *d_order = db.get<int32_t>(n), *d_tmp = db.get<int32_t>(demgb::scan_tmp_size(std::max(cells, n + 1)));
-        int32_t *d_sel = db.get<int32_t>((size_t)n * max_bonds), *d_count = db.get<int32_t>(n);
-        int32_t *d_base = db.get<int32_t>(n + 1);
-        if (!d_pos || !d_r || !d_keys || !d_cnt || !d_start || !d_order || !d_tmp || !d_sel || !d_count || !d_base) {
+        DevBlock first, second;
+        float2 *d_pos;
+        float *d_r;
+        int32_t *d_keys, *d_cnt, *d_start, *d_order, *d_tmp, *d_sel, *d_count, *d_base, *d_in, *d_in_start, *d_sc;
+        if (!first.carve([&](Carve &c) {
+                d_pos = c.take<float2>(n);
+                d_r = c.take<float>(n);
+                d_keys = c.take<int32_t>(n);
+                d_cnt = c.take<int32_t>(cells);
+                d_start = c.take<int32_t>((size_t)cells + 1);
+                d_order = c.take<int32_t>(n);
+                d_tmp = c.take<int32_t>(demgb::scan_tmp_size(std::max(cells, n + 1)));
+                d_sel = c.take<int32_t>((size_t)n * max_bonds);
+                d_count = c.take<int32_t>(n);
+                d_base = c.take<int32_t>((size_t)n + 1);
+                d_in = c.take<int32_t>(n);
+                d_in_start = c.take<int32_t>((size_t)n + 1);
+                d_sc = c.take<int32_t>((size_t)demgb::SORT_GRID_MAX * demgb::SORT_BINS);
+            }))
             rc = bfail(DEM_E_OOM, "device allocation failed");
-        }
         const int T = 256, G = (n + T - 1) / T;
         if (rc == DEM_OK) {
             cudaMemcpyAsync(d_pos, pos, sizeof(float2) * n, cudaMemcpyHostToDevice, st);
@@ -271,18 +340,27 @@ int dem_generate_bonds(const float *pos, const float *radii, int32_t n, int32_t 
                 rc = bfail(DEM_E_CAPACITY, "bonds_cap is smaller than the bond count written to *n_bonds");
         }
         if (rc == DEM_OK) {
-            int32_t *d_bonds = db.get<int32_t>(3 * (size_t)total), *d_bi = db.get<int32_t>(total);
-            int32_t *d_bj = db.get<int32_t>(total), *d_in = db.get<int32_t>(n), *d_in_start = db.get<int32_t>(n + 1);
-            int32_t *d_list = db.get<int32_t>(total), *d_v2 = db.get<int32_t>(total);
-            uint32_t *d_k1 = db.get<uint32_t>(total), *d_k2 = db.get<uint32_t>(total);
-            int32_t *d_sc = db.get<int32_t>((size_t)demgb::SORT_GRID_MAX * demgb::SORT_BINS);
-            int32_t *d_contacts = db.get<int32_t>((size_t)n * K * 6);
-            if (!d_bonds || !d_bi || !d_bj || !d_in || !d_in_start || !d_list || !d_v2 || !d_k1 || !d_k2 ||
-                !d_sc || !d_contacts) {
+            int32_t *d_bi, *d_bj, *d_list, *d_v2, *d_contacts;
+            uint32_t *d_k1, *d_k2;
+            if (!second.carve([&](Carve &c) {
+                    d_bi = c.take<int32_t>(total);
+                    d_bj = c.take<int32_t>(total);
+                    d_list = c.take<int32_t>(total);
+                    d_v2 = c.take<int32_t>(total);
+                    d_k1 = c.take<uint32_t>(total);
+                    d_k2 = c.take<uint32_t>(total);
+                    d_contacts = c.take<int32_t>((size_t)n * K * 6);
+                })) {
                 rc = bfail(DEM_E_OOM, "device allocation failed");
             } else {
                 cudaMemsetAsync(d_in, 0, sizeof(int32_t) * n, st);
-                k_bg_write<<<G, T, 0, st>>>(n, max_bonds, d_sel, d_count, d_base, d_bonds, d_bi, d_bj, d_in);
+                k_bg_write<<<G, T, 0, st>>>(n, max_bonds, d_sel, d_count, d_base, d_bi, d_bj, d_in);
+                std::vector<int32_t> bi(total), bj(total);
+                if (total > 0) {
+                    cudaMemcpyAsync(bi.data(), d_bi, sizeof(int32_t) * total, cudaMemcpyDeviceToHost, st);
+                    cudaMemcpyAsync(bj.data(), d_bj, sizeof(int32_t) * total, cudaMemcpyDeviceToHost, st);
+                }
+                const cudaError_t se = cudaStreamSynchronize(st);  // the host's part starts with these
                 demgb::launch_exclusive_scan(d_in, d_in_start, n, d_tmp, st);
                 if (total > 0) {
                     // incoming bonds of every particle in ascending bond number:
@@ -305,28 +383,15 @@ int dem_generate_bonds(const float *pos, const float *radii, int32_t n, int32_t 
                         prev.val = ov;
                     }
                 }
-                k_bg_slots<<<G, T, 0, st>>>(n, max_bonds, d_count, d_base, d_sel, d_in_start, d_list, d_bi,
-                                            d_contacts);
-                std::vector<int32_t> bi(total), bj(total);
-                if (total > 0) {
-                    cudaMemcpyAsync(bonds, d_bonds, sizeof(int32_t) * 3 * (size_t)total, cudaMemcpyDeviceToHost, st);
-                    cudaMemcpyAsync(bi.data(), d_bi, sizeof(int32_t) * total, cudaMemcpyDeviceToHost, st);
-                    cudaMemcpyAsync(bj.data(), d_bj, sizeof(int32_t) * total, cudaMemcpyDeviceToHost, st);
-                }
+                k_bg_slots<<<(n + BG_SLOTS - 1) / BG_SLOTS, BG_SLOTS, 0, st>>>(n, max_bonds, d_count, d_base, d_sel,
+                                                                              d_in_start, d_list, d_bi, d_contacts);
                 cudaMemcpyAsync(contacts, d_contacts, sizeof(int32_t) * (size_t)n * K * 6, cudaMemcpyDeviceToHost, st);
-                if (cudaStreamSynchronize(st) != cudaSuccess) {
-                    rc = bfail(DEM_E_CUDA, cudaGetErrorString(cudaGetLastError()));
-                } else {
-                    // length = (dx*dx + dy*dy)^0.5, angle = atan2(dx / |d|, dy / |d|)
-                    // (state.rs:309-313)
-                    for (int32_t b = 0; b < total; ++b) {
-                        const int i = bi[b], j = bj[b];
-                        const float dx = pos[2 * j] - pos[2 * i], dy = pos[2 * j + 1] - pos[2 * i + 1];
-                        const float mag = std::pow(dx * dx + dy * dy, 0.5f);
-                        const float ang = std::atan2(dx / mag, dy / mag);
-                        std::memcpy(&bonds[3 * (size_t)b + 1], &ang, 4);
-                        std::memcpy(&bonds[3 * (size_t)b + 2], &mag, 4);
-                    }
+                // behind the sort, the slots and their copy
+                if (se == cudaSuccess) bond_records(pos, bi.data(), bj.data(), total, bonds);
+                const cudaError_t e = cudaStreamSynchronize(st);
+                if (se != cudaSuccess || e != cudaSuccess) {
+                    rc = bfail(DEM_E_CUDA, cudaGetErrorString(se != cudaSuccess ? se : e));
+                    cudaGetLastError();
                 }
             }
         }
