@@ -29,15 +29,27 @@ constexpr int PK_MAX_THREADS = 1024;
 
 __device__ __forceinline__ float len2f(float x, float y) { return sqrtf(x * x + y * y); }
 
-// cell range of the particle's AABB in the reference grid (2D_LOM.wgsl:167-178);
-// i32() is truncation toward zero, saturating (cvt.rzi).
+// i32(v / cs) (truncation toward zero, saturating: cvt.rzi) with inv the
+// rounded reciprocal of cs.  Only a quotient's integer part is wanted, and
+// v * inv has the same one unless an integer lies within the two products'
+// roundings (1.5 x 2^-23 of the value; the reciprocal's, this product's and
+// the quotient's own): the division is taken only then -- about once in 10^4
+// on a grid of 150 buckets -- and when inv is NaN (cs outside the range in
+// which its reciprocal has full precision) or anything overflows.
+__device__ __forceinline__ int bucket_of(float v, float cs, float inv) {
+    const float t = v * inv;
+    if (fabsf(t - rintf(t)) > fabsf(t) * 2.4e-7f) return __float2int_rz(t);
+    return __float2int_rz(v / cs);
+}
+
+// cell range of the particle's AABB in the reference grid (2D_LOM.wgsl:167-178)
 __device__ __forceinline__ void ref_range(const ScenePar &P, float px, float py, float r, int &x0,
                                           int &x1, int &y0, int &y1) {
     float left = px - r, right = px + r, bottom = py - r, top = py + r;
-    int a = __float2int_rz((left - P.ref_base_x) / P.ref_cs);
-    int b = __float2int_rz((right - P.ref_base_x) / P.ref_cs);
-    int c = __float2int_rz((P.ref_base_y - top) / P.ref_cs);
-    int d = __float2int_rz((P.ref_base_y - bottom) / P.ref_cs);
+    int a = bucket_of(left - P.ref_base_x, P.ref_cs, P.ref_inv);
+    int b = bucket_of(right - P.ref_base_x, P.ref_cs, P.ref_inv);
+    int c = bucket_of(P.ref_base_y - top, P.ref_cs, P.ref_inv);
+    int d = bucket_of(P.ref_base_y - bottom, P.ref_cs, P.ref_inv);
     x0 = a > 0 ? a : 0;
     x1 = b < P.ref_w - 1 ? b : P.ref_w - 1;
     y0 = c > 0 ? c : 0;
@@ -197,6 +209,18 @@ __device__ __forceinline__ F3 linear_model(const ScenePar &P, float2 kns, float4
 }
 
 __device__ __forceinline__ int sign_i32(float x) { return x > 0.0f ? 1 : (x < 0.0f ? -1 : 0); }
+
+// Whether a parallel bond plainly holds: the tear test Fn / A - X / I < -sn or
+// T / A > ss (2D_Simulation.wgsl:318-319) with both sides multiplied by A I
+// and A, and room for every rounding on either side (each below 2^-22 of the
+// terms, the room 1e-5 of them and 1e-4), so that three divisions are taken
+// only close to a tear.  False also where a product could leave the range in
+// which its relative error is a rounding.
+__device__ __forceinline__ bool bond_holds(float Fn, float X, float T, float A, float I, float sn, float ss) {
+    const float f = Fn * I, x = X * A, lim = (sn * A) * I, sh = ss * A;
+    return I >= 1e-12f && lim >= 1e-25f && sh >= 1e-25f &&
+           f - x > 1e-5f * ((fabsf(f) + fabsf(x)) + lim) - lim && T < 0.9999f * sh;
+}
 
 __device__ __forceinline__ void record_break(const DevWorld &w, const ScenePar &P, int scene,
                                              long long step, int bond_global, int code, int a_int,
@@ -1741,9 +1765,9 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Own 
                 float bend = ((-kn) * I) * thb;
                 bend = bend < 0.0f ? -bend : bend;
                 const float abtf = btf < 0.0f ? -btf : btf;
-                if (U.p.bonds_tear == 1 &&
-                    ((Fn / A) - (U.p.moment_contribution_factor * (bend * Rr)) / I < -sn ||
-                     abtf / A > ss)) {
+                const float X = U.p.moment_contribution_factor * (bend * Rr);
+                if (U.p.bonds_tear == 1 && !bond_holds(Fn, X, abtf, A, I, sn, ss) &&
+                    ((Fn / A) - X / I < -sn || abtf / A > ss)) {
                     const int code = -10 + sign_i32(nd);
                     record_break(w, P, s, o.step(w), bg, code, i, b);
                     o.broke();

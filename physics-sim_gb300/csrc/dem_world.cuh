@@ -65,6 +65,7 @@ struct ScenePar {
     float xW, yH;          // hor_bound / 2, vert_bound / 2 (2D_LOM.wgsl:105-106)
     // reference bucket grid: defines which pairs are candidates and in which order
     float ref_cs, ref_base_x, ref_base_y;
+    float ref_inv;         // 1 / ref_cs rounded, NaN where that loses precision (bucket_of)
     int32_t ref_w, ref_h;
     // search grid (centre-binned, complete for every pair the reference grid can find)
     float g_x0, g_y0, g_inv, g_cs;

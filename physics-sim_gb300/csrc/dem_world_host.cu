@@ -814,6 +814,7 @@ void World::fill_par(SceneHost &h) {
     P.xW = h.params.hor_bound / 2.0f;
     P.yH = h.params.vert_bound / 2.0f;
     P.ref_cs = h.grid.cell_size;
+    P.ref_inv = P.ref_cs >= 1e-30f && P.ref_cs <= 1e30f ? 1.0f / P.ref_cs : std::numeric_limits<float>::quiet_NaN();
     P.ref_w = h.grid.w;
     P.ref_h = h.grid.h;
     P.ref_base_x = ((-h.grid.cell_size) * (float)h.grid.w) * 0.5f;
