@@ -1527,33 +1527,24 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Own 
             // unrolled tests stop at the longest list among the warp's lanes
             // here (a warp-uniform exit: sparse warps skip the empty tail).
             const int lmax = __reduce_max_sync(__activemask(), lc);
-            if (Own::RESIDENT) {
-                // few warps hide a gather's latency here: half a list in flight at once
+            // Gathers in flight at once.  k_steps' few warps hide no latency
+            // by themselves and have the registers for half a list; k_narrow
+            // has room for two (4.2 M-particle impact scene 377 -> 371 us a
+            // step; three 380, four 395 with its spills); k_interact, which
+            // spills already, gains nothing from two.
+            constexpr int BATCH = Own::RESIDENT ? 8 : PART == 1 ? 2 : 1;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (8 * h > lmax) break;
-                    float4 pb[8];
+            for (int k0 = 1; k0 <= NL; k0 += BATCH) {
+                if (k0 > lmax) break;
+                float4 pb[BATCH];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const int k = 8 * h + q;
-                        if (k > 0 && k <= lc) pb[q] = o.partner(w, i + nl_entry(la, lb, k));
-                    }
+                for (int q = 0; q < BATCH; ++q)
+                    if (k0 + q <= lc && k0 + q <= NL) pb[q] = o.partner(w, i + nl_entry(la, lb, k0 + q));
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const int k = 8 * h + q;
-                        if (k > 0 && k <= lc && touching(pa, pb[q]) && shares_bucket(ca, __float_as_uint(pb[q].w)))
-                            pass |= 1u << k;
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int k = 1; k <= NL; ++k) {
-                    if (k > lmax) break;
-                    if (k <= lc) {
-                        const float4 pb = o.partner(w, i + nl_entry(la, lb, k));
-                        if (touching(pa, pb) && shares_bucket(ca, __float_as_uint(pb.w))) pass |= 1u << k;
-                    }
-                }
+                for (int q = 0; q < BATCH; ++q)
+                    if (k0 + q <= lc && k0 + q <= NL && touching(pa, pb[q]) &&
+                        shares_bucket(ca, __float_as_uint(pb[q].w)))
+                        pass |= 1u << (k0 + q);
             }
             if (wide_range(ca)) {  // the range limits, checked on every partner
                 unsigned rank;
