@@ -131,20 +131,52 @@ struct F3 {
     float x, y, z;
 };
 
+// (float)(sqrt(dx^2 + dy^2) - (lh + ll)) with the differences, the root and
+// the subtraction in double (lh + ll exact in double), the F64 branch of both
+// distances.  Double precision runs at 1/64 of the float rate here, so the
+// value is first formed in pairs of floats, to 2^-42 of the root (differences
+// and squares exact to a pair, one Newton correction of the float root whose
+// residual is exact), and taken if moving it by that much either way rounds
+// to the same float: the double evaluation, whose own roundings are below
+// 2^-51, then rounds to it too.  Otherwise (one evaluation in ~4,000, or
+// operands outside the range in which the pairs are exact) the expression is
+// evaluated as written.  30,011-particle bed, F64 distances: 13.0 -> 10.0 us a
+// step.
+__device__ __forceinline__ float gap_f64(float4 pa, float4 pb, float lh, float ll) {
+    const auto two_sum = [](float x, float y, float &err) {  // x + y = sum + err (Knuth)
+        const float sum = x + y, yy = sum - x, xx = sum - yy;
+        err = (x - xx) + (y - yy);
+        return sum;
+    };
+    float xl, yl, sl, gl, rest;
+    const float xh = two_sum(pa.x, -pb.x, xl), yh = two_sum(pa.y, -pb.y, yl);
+    const float px = xh * xh, py = yh * yh;
+    const float ex = __fmaf_rn(xh, xh, -px) + 2.0f * (xh * xl), ey = __fmaf_rn(yh, yh, -py) + 2.0f * (yh * yl);
+    const float s0 = two_sum(px, py, sl);
+    sl = sl + (ex + ey);
+    const float s1 = s0 + sl, s2 = sl - (s1 - s0);
+    const float root = sqrtf(s1);
+    const float fix = (__fmaf_rn(-root, root, s1) + s2) * (0.5f / root);
+    const float g0 = two_sum(root, -lh, gl);
+    gl = gl + (fix - ll);
+    const float g = two_sum(g0, gl, rest);
+    const float err = root * 2.4e-13f;
+    if (root > 1e-9f && root < 1e9f && g + (rest + err) == g && g + (rest - err) == g) return g;
+    const double dx = (double)pa.x - (double)pb.x, dy = (double)pa.y - (double)pb.y;
+    return (float)(sqrt(dx * dx + dy * dy) - ((double)lh + (double)ll));
+}
+
 // distance2 (2D_Simulation.wgsl:273-284): |pa-pb| - length, F64 branch optional
 __device__ __forceinline__ float distance2(int use_f64, float4 pa, float4 pb, float length) {
-    if (use_f64) {
-        double dx = (double)pa.x - (double)pb.x, dy = (double)pa.y - (double)pb.y;
-        return (float)(sqrt(dx * dx + dy * dy) - (double)length);
-    }
+    if (use_f64) return gap_f64(pa, pb, length, 0.0f);
     float dx = pa.x - pb.x, dy = pa.y - pb.y;
     return len2f(dx, dy) - length;
 }
 // distance (2D_Simulation.wgsl:264-271): the F64 branch sums the radii in double
 __device__ __forceinline__ float distance1(int use_f64, float4 pa, float4 pb) {
     if (use_f64) {
-        double dx = (double)pa.x - (double)pb.x, dy = (double)pa.y - (double)pb.y;
-        return (float)(sqrt(dx * dx + dy * dy) - ((double)pa.z + (double)pb.z));
+        const float lh = pa.z + pb.z, zz = lh - pa.z;
+        return gap_f64(pa, pb, lh, (pa.z - (lh - zz)) + (pb.z - zz));
     }
     float dx = pa.x - pb.x, dy = pa.y - pb.y;
     return len2f(dx, dy) - (pa.z + pb.z);

@@ -48,3 +48,56 @@ def test_bond_holds_only_where_the_tear_test_fails(seed):
     tears = (((Fn / A).astype(F) - (X / I).astype(F)).astype(F) < -sn) | ((T / A).astype(F) > ss)
     assert not np.any(holds & tears)
     assert 0.02 < holds.mean() < 0.9 and tears.mean() > 0.1
+
+
+def _fma(x, y, z):
+    """float32 fused multiply-add: the product is exact in float64, and so is
+    the sum here, whose terms cancel (gap_f64 takes residuals of x*y near -z)."""
+    return (x.astype(np.float64) * y.astype(np.float64) + z.astype(np.float64)).astype(F)
+
+
+def _two_sum(x, y):
+    s = (x + y).astype(F)
+    yy = (s - x).astype(F)
+    xx = (s - yy).astype(F)
+    return s, ((x - xx).astype(F) + (y - yy).astype(F)).astype(F)
+
+
+@pytest.mark.parametrize("seed", range(8))
+def test_gap_f64_rounds_like_double(seed):
+    rng = np.random.default_rng(seed)
+    n = 1_000_000
+    span = 10.0 ** rng.uniform(-4, 5)
+    ax, ay = rng.uniform(-span, span, (2, n)).astype(F)
+    ang, d = rng.uniform(0, 2 * np.pi, n), 10.0 ** rng.uniform(-3, 1, n)
+    bx, by = (ax + d * np.cos(ang)).astype(F), (ay + d * np.sin(ang)).astype(F)
+    dx, dy = ax.astype(np.float64) - bx, ay.astype(np.float64) - by
+    L = np.sqrt(dx * dx + dy * dy)
+    # lengths from the distance itself, a few roundings off, to twice it
+    lh = (L * (1.0 + rng.choice([-1, 1], n) * 2.0 ** rng.uniform(-26, 0, n))).astype(F)
+    ll = np.zeros(n, F)
+    if seed % 2:  # a sum of two radii in double
+        ra = (lh * rng.uniform(0.1, 0.9, n)).astype(F)
+        rb = (lh - ra).astype(F)
+        lh, ll = _two_sum(ra, rb)
+    want = (L - (lh.astype(np.float64) + ll)).astype(F)
+    xh, xl = _two_sum(ax, -bx)
+    yh, yl = _two_sum(ay, -by)
+    px, py = (xh * xh).astype(F), (yh * yh).astype(F)
+    ex = (_fma(xh, xh, -px) + (F(2) * (xh * xl).astype(F)).astype(F)).astype(F)
+    ey = (_fma(yh, yh, -py) + (F(2) * (yh * yl).astype(F)).astype(F)).astype(F)
+    s0, sl = _two_sum(px, py)
+    sl = (sl + (ex + ey).astype(F)).astype(F)
+    s1 = (s0 + sl).astype(F)
+    s2 = (sl - (s1 - s0).astype(F)).astype(F)
+    with np.errstate(divide="ignore", invalid="ignore"):
+        root = np.sqrt(s1)
+        fix = ((_fma(-root, root, s1) + s2).astype(F) * (F(0.5) / root).astype(F)).astype(F)
+        g0, gl = _two_sum(root, -lh)
+        gl = (gl + (fix - ll).astype(F)).astype(F)
+        g, rest = _two_sum(g0, gl)
+        err = (root * F(2.4e-13)).astype(F)
+        taken = (root > F(1e-9)) & (root < F(1e9)) & ((g + (rest + err).astype(F)).astype(F) == g) & \
+            ((g + (rest - err).astype(F)).astype(F) == g)
+    assert np.array_equal(g[taken], want[taken])
+    assert taken.mean() > 0.5
