@@ -405,6 +405,15 @@ __device__ __forceinline__ bool chunk_live(const DevWorld &w, int i) {
     return w.live == nullptr || __ldg(&w.live[i >> 7]) != 0;
 }
 
+// a candidate list's first word h0 (count and flags) and the slot word's NL_LIVE bit
+__device__ __forceinline__ void list_head(const DevWorld &w, int i, int16_t *h, int h0) {
+    h[0] = (int16_t)h0;
+    w.cmask[i] = CM_STALE;  // the match word described the old list
+    const uint32_t sm = w.smask[i];
+    const uint32_t nsm = h0 != 0 ? (sm | NL_LIVE) : (sm & ~NL_LIVE);
+    if (nsm != sm) w.smask[i] = nsm;
+}
+
 #ifndef DEM_STEP_DEVICE_CODE  // dem_steps.cu includes this file for the step's device functions alone
 // With w.ticket the kernel's last warp sets the rebuild conditional; without
 // it (large worlds, where thousands of fenced ticket atomics cost more than a
@@ -908,15 +917,6 @@ void launch_reorder(const DevWorld &w, const DevWorld &spare, int block, cudaStr
 // skin/2.  More than NL candidates, or one farther than an int16 offset can
 // reach: the particle searches the cell table (built in the same rebuild) at
 // every step instead.
-// the list's first word h0 (count and flags) and the slot word's NL_LIVE bit
-__device__ __forceinline__ void list_head(const DevWorld &w, int i, int16_t *h, int h0) {
-    h[0] = (int16_t)h0;
-    w.cmask[i] = CM_STALE;  // the match word described the old list
-    const uint32_t sm = w.smask[i];
-    const uint32_t nsm = h0 != 0 ? (sm | NL_LIVE) : (sm & ~NL_LIVE);
-    if (nsm != sm) w.smask[i] = nsm;
-}
-
 // Candidate lists one particle a thread in internal order, the cell table's
 // cells read from global memory: the form for sparse worlds (about one
 // particle a search cell or fewer, where a block's particles span too many
@@ -1353,9 +1353,11 @@ struct HbmOwn {
     uint32_t m, mask;
     float4 pa;
     int N, i;
-    __device__ __forceinline__ HbmOwn(const DevWorld &w, int i_) : N(w.N), i(i_) {
+    __device__ __forceinline__ HbmOwn(const DevWorld &w, int i_) : HbmOwn(w, i_, w.pr, w.dp) {}
+    __device__ __forceinline__ HbmOwn(const DevWorld &w, int i_, const float4 *pr, const float4 *dp)
+        : N(w.N), i(i_) {
         m = w.meta[i];
-        pa = w.pr[i];
+        pa = pr[i];
         mask = w.smask[i];
         if (PART != 1) {
             prefetch_l1(&w.vw[i]);
@@ -1367,7 +1369,7 @@ struct HbmOwn {
             prefetch_l1(&w.nl[2 * (size_t)i]);
             prefetch_l1(&w.cmask[i]);
         }
-        if (PART != 1 && (mask & SLOT_BITS)) prefetch_l1(&w.dp[i]);
+        if (PART != 1 && (mask & SLOT_BITS)) prefetch_l1(&dp[i]);
         for (uint32_t left = PART != 1 ? mask & SLOT_BITS : 0u; left; left &= left - 1) {
             const int j = __ffs(left) - 1;
             prefetch_l1(&w.s_b[j * N + i]);

@@ -275,6 +275,7 @@ struct RunRecord {
     float *out = nullptr;
 };
 int device_sms();  // SMs of the current device
+constexpr int SWEEP_THREADS = 1024;  // block size of the worlds whose particles exceed the threads; they record no data
 int steps_block(int n);
 void launch_run_begin(const DevWorld &w, int todo, const RunRecord &rec, cudaStream_t st);
 cudaError_t launch_steps(const DevWorld &w, int block, cudaStream_t st, cudaGraphConditionalHandle more,

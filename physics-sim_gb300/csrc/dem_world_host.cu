@@ -2362,7 +2362,7 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
     const int chunk = (int)std::max<long long>(1, std::min<long long>(n_steps, (1LL << 24) / per));
     // a resident run records inside its kernel, which looks up each particle's
     // row; else a gather after every step takes the list of recorded particles
-    const bool resident = runs_resident();
+    const bool resident = runs_resident() && run_block != SWEEP_THREADS;
     std::vector<int32_t> row_of;
     if (resident) {
         row_of.assign((size_t)h.n, -1);

@@ -24,8 +24,10 @@ def shaken_bed(n, seed, speed=8.0, spacing=2.05):
 
 
 # one particle; a warp and a block and one more; the last size of 128, of 256
-# and of 512 threads on 152 SMs and the first beyond each
-@pytest.mark.parametrize("n", [1, 33, 128, 129, 2500, 19456, 19457, 38912, 38913, 77824, 77825])
+# and of 512 threads on 152 SMs and the first beyond each; the last size of a
+# sweep of one particle a thread, of two, and the first of a launch a step
+@pytest.mark.parametrize("n", [1, 33, 128, 129, 2500, 19456, 19457, 38912, 38913, 77824, 77825, 155648, 155649,
+                               311296, 311297])
 def test_sizes_bit_exact(n):
     sc, p, ext = shaken_bed(n, n % 97)
     ref = copy_scene(sc)
@@ -40,12 +42,13 @@ def test_sizes_bit_exact(n):
         assert st["reorders"] >= 2, "no list was rebuilt within a run"
 
 
-@pytest.mark.parametrize("cell_factor,every", [(0.7, 0), (1.0, 1), (1.0, 2)])
-def test_lists_longer_than_their_capacity(cell_factor, every):
+@pytest.mark.parametrize("n,cell_factor,every", [(700, 0.7, 0), (700, 1.0, 1), (700, 1.0, 2), (80000, 1.0, 0),
+                                                 (80000, 0.7, 2)])
+def test_lists_longer_than_their_capacity(n, cell_factor, every):
     """Disks so crowded that some have more than 15 candidates, which search
     their cells at every step; 3 x 3 and 5 x 5 cells, lists from chains and
     from the sorted rebuild."""
-    sc, p, _ = shaken_bed(700, 5, speed=4.0, spacing=1.1)
+    sc, p, _ = shaken_bed(n, 5, speed=4.0, spacing=1.1)
     ref = copy_scene(sc)
     with dem.Context(copy_scene(sc), p, search_cell_factor=cell_factor, reorder_every=every) as ctx:
         for steps in (25, 30):
@@ -56,7 +59,7 @@ def test_lists_longer_than_their_capacity(cell_factor, every):
     assert st["list_overflows"] > 0 and st["reorders"] >= 2
 
 
-@pytest.mark.parametrize("chains,length", [(3, 30), (16, 40)])
+@pytest.mark.parametrize("chains,length", [(3, 30), (16, 40), (700, 150)])
 def test_breaks_cross_blocks(chains, length):
     """Bonds break on both sides of block borders; breaks are seen a step later."""
     sc, p, ext = dem_scenes.c1_chains(chains=chains, length=length, seed=9, pull_velocity=25.0)
@@ -71,15 +74,16 @@ def test_breaks_cross_blocks(chains, length):
         assert events > 0 and len(ctx.break_events()) == events
 
 
-def test_schedules_settings_and_the_way_out():
+@pytest.mark.parametrize("n", [1500, 79000])
+def test_schedules_settings_and_the_way_out(n):
     """Narrow phase every 4th step, settings changed between calls, positions
     set from outside, a step by plain launches between runs (which needs the
     sorted cell table again), and a record in between."""
-    sc, p, ext = shaken_bed(1500, 3)
+    sc, p, ext = shaken_bed(n, 3)
     p = dict(p, collision_interval=4)
     ref = copy_scene(sc)
-    sel = np.zeros(1500, np.int32)
-    sel[[0, 7, 1499]] = 1
+    sel = np.zeros(n, np.int32)
+    sel[[0, 7, n - 1]] = 1
     with dem.Context(copy_scene(sc), p, **ext) as ctx:
         def both(steps):
             ctx.step(steps)
@@ -108,9 +112,10 @@ def test_schedules_settings_and_the_way_out():
 
 
 @pytest.mark.parametrize("shared", [True, False])
-def test_batches_bit_exact(shared):
+@pytest.mark.parametrize("most", [2000, 100000])
+def test_batches_bit_exact(shared, most):
     """Scenes with shared settings and with settings of their own."""
-    items = [shaken_bed(n, k) for k, n in enumerate((5, 200, 1, 431, 2000))]
+    items = [shaken_bed(n, k) for k, n in enumerate((5, 200, 1, 431, most))]
     for k, it in enumerate(items):
         it[1]["gravity_acc"] = 1.0 if shared else 1.0 + 0.25 * k
     refs = [copy_scene(it[0]) for it in items]
@@ -123,11 +128,13 @@ def test_batches_bit_exact(shared):
             assert_same_state(b.download(k), refs[k], "scene %d: " % k)
 
 
-def test_horizons_end_within_a_run():
-    """Served scenes that stop at their own steps inside one advance."""
+@pytest.mark.parametrize("arena", [2000, 40000])
+def test_horizons_end_within_a_run(arena):
+    """Served scenes that stop at their own steps inside one advance; arenas
+    with a thread and with a sweep for every particle's place."""
     items = [shaken_bed(n, 20 + k) for k, n in enumerate((300, 77, 900))]
     horizons = (25, 70, 41)
-    with dem.Server(max_active_particles=2000, max_scenes=8) as sv:
+    with dem.Server(max_active_particles=arena, max_scenes=8) as sv:
         ids = [sv.submit(sc, p, h, **e) for (sc, p, e), h in zip(items, horizons)]
         done = []
         while len(done) < len(ids):
