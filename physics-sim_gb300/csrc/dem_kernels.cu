@@ -1415,6 +1415,7 @@ struct HbmOwn {
     __device__ __forceinline__ float4 partner_disp(const DevWorld &w, int b) const { return __ldg(&w.dp[b]); }
     __device__ __forceinline__ int bond_status(const DevWorld &w, int g) const { return w.b_status[g]; }
     __device__ __forceinline__ void broke() {}
+    __device__ __forceinline__ unsigned lanes_of_step() const { return __activemask(); }
     __device__ __forceinline__ void record(const DevWorld &, float4, float, float, float, float) {}
     // the rest of the particle's own record
     __device__ __forceinline__ float2 stiffness(const DevWorld &w, int, int at) const { return __ldg(&w.pair[at]); }
@@ -1496,6 +1497,15 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Own 
         if (FUSE) o.stay(w);
         return;
     }
+    // Whether the force loop takes its slots in rounds, the warp's lanes brought
+    // together at each (the compiler need not, and a group of lanes that lags
+    // behind runs the rest of the loop on its own).  It pays where a slot's
+    // arithmetic is long and its lanes part: the split kernels of dense bonded
+    // scenes (4.2 M-particle impact scene 371 -> 360 us a step) and the F64
+    // distances in k_steps (30,011-particle bed 10.4 -> 9.8); it costs 1 to 10 %
+    // elsewhere.
+    constexpr bool ROUNDS = PART == 2 || (Own::RESIDENT && FORM == -1);
+    const unsigned lanes = ROUNDS ? o.lanes_of_step() : 0u;
     const uint32_t before = mask;
     const int bonds_model = FORM == 0 ? 0 : FORM == 3 ? 3 : U.p.bonds;
     constexpr bool MAY_F64 = FORM == -1;
@@ -1729,7 +1739,12 @@ __device__ __forceinline__ void interact_particle(const DevWorld &w, int i, Own 
     Acc3 acc = {0.0f, 0.0f, 0.0f};
     uint32_t left = mask & SLOT_BITS;
     if (Own::RESIDENT && changed && left) ahead = fetch(__ffs(left) - 1);
-    while (left) {
+    const int rounds = ROUNDS ? __reduce_max_sync(lanes, __popc(left)) : 0;
+    for (int round = 0; ROUNDS ? round < rounds : left != 0u; ++round) {
+        if (ROUNDS) {
+            __syncwarp(lanes);
+            if (!left) continue;
+        }
         const int j = __ffs(left) - 1;
         left &= left - 1;
         const SlotIn in = Own::RESIDENT ? ahead : fetch(j);
