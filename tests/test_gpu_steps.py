@@ -146,3 +146,32 @@ def test_horizons_end_within_a_run(arena):
             ref = copy_scene(sc)
             oracle.step(ref, p, h)
             assert_same_state(got, ref, "horizon %d: " % h)
+
+
+def test_worlds_on_threads_of_their_own():
+    """Contexts of every kind of run stepped at the same time."""
+    import threading
+
+    todo = []
+    for n, seed in ((30011, 1), (4000, 2), (100000, 3), (128, 4), (700, 5)):
+        sc, p, _ = shaken_bed(n, seed)
+        ref = copy_scene(sc)
+        oracle.step(ref, p, 60)
+        todo.append((sc, p, ref, []))
+
+    def work(sc, p, ref, got):
+        for _ in range(3):
+            with dem.Context(copy_scene(sc), p) as ctx:
+                for _ in range(4):
+                    ctx.step(15)
+                got.append(ctx.download())
+
+    threads = [threading.Thread(target=work, args=t) for t in todo]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for sc, _, ref, got in todo:
+        assert len(got) == 3
+        for g in got:
+            assert_same_state(g, ref, "%d particles: " % sc["radii"].size)
