@@ -89,7 +89,10 @@ typedef struct dem_ext {
     const float *bond_normal_strength;/* optional per-bond strengths [n_bonds]; NULL = global setting */
     const float *bond_shear_strength;
     int32_t diagnostics;              /* 1: maintain data[7n] every step as the reference does */
-    int32_t reorder_interval;         /* steps per captured CUDA graph; 0 = library default (35) */
+    int32_t reorder_interval;         /* steps per captured CUDA graph; 0 = library default (35).  Worlds
+                                         of up to 311,296 particles, none of them large, take a step
+                                         call in one kernel: reorder_interval, block_size,
+                                         split_narrow and unfused_lom have no effect there */
     int32_t block_size;               /* threads per block for particle kernels; 0 = default */
     float search_cell_factor;         /* search-grid cell / (2 r_max + skin), in [0.5, inf); 0 = default
                                          1.0.  Below 1 the cell searches span 5 x 5 cells instead of
@@ -112,7 +115,8 @@ typedef struct dem_ext {
                                          page tables (Grace), else through a page-locked block; 1: always
                                          through the page-locked block */
     int32_t reorder_every;            /* rebuilds per reorder of the particle arrays into cell order; 0 =
-                                         default: 3 in a single-scene context, 8 in batches and servers.
+                                         default: 3 in a single-scene context, 8 in batches and servers,
+                                         32 where a step call is one kernel (records in cache anyway).
                                          Every rebuild sorts by cell and rebuilds the candidate
                                          lists; the reorder only restores memory locality, which particles
                                          lose slowly (they move a skin between rebuilds, a cell takes
@@ -172,7 +176,9 @@ typedef struct dem_stats {
                                    pending-break capacity; 2 a touching pair whose first shared bucket
                                    ranks beyond 15 in the scan order, or an AABB 31 or more buckets
                                    wide (the bucket grid is much finer than the particles); 4 a large
-                                   particle touching more than 2048 particles at once */
+                                   particle touching more than 2048 particles at once; 8 a step
+                                   kernel's wait for its own blocks ran out of time (reported as
+                                   DEM_E_TIMEOUT by the next call that waits) */
     int32_t reserved;
     int64_t kernel_launches;    /* kernels this library launched on the context's stream */
     int64_t list_overflows;     /* particles whose candidates exceeded the list (searched the cells) */

@@ -1837,11 +1837,11 @@ int World::capture_run(cudaGraphExec_t *out) {
     return DEM_OK;
 }
 
-// Whether a step call is one run of k_steps.  Every world whose particles
-// fit one a thread takes it (a launch a step -> a run, microseconds a step:
-// 128 bonded particles 19.4 -> 4.9, 4,096 falling 13.8 -> 3.7, 16,384 bonded
-// 18.2 -> 6.9, a 30,011-particle bed with F64 distances 35.9 -> 15, its FP32
-// form of 70,000 33.6 -> 13.7); k_big_narrow is a launch of its own.
+// Whether a step call is one run of k_steps or k_sweep.  Every world whose
+// particles fit two a thread takes it (a launch a step -> a run, microseconds
+// a step: 128 bonded particles 19.4 -> 4.2, 4,096 falling 13.8 -> 2.7, 16,384
+// bonded 18.2 -> 5.7, a 30,011-particle bed with F64 distances 35.9 -> 9.8, a
+// 262,144-particle bed 44.3 -> 31.4); k_big_narrow is a launch of its own.
 bool World::runs_resident() const { return use_graphs && !timing && !has_bigs && run_block > 0; }
 
 // one run of n_steps, recording the datum of the particles in rec.rows
@@ -1905,8 +1905,9 @@ void World::update_param_source() {
 
 // One Simulation kernel or two.  Where particles have many contacts and some
 // are bonded, the single kernel's register cap spills inside the force loop
-// and the split pays (4.2 M-particle impact bed 469 -> 395 us a step, its
-// 262,145-particle crop 68 -> 62); without bonds, or with fewer contacts a
+// and the split pays (4.2 M-particle impact bed 469 -> 395 us a step before
+// the split kernels' own later steps, 356 now; its 262,145-particle crop
+// 68 -> 62); without bonds, or with fewer contacts a
 // particle, the second read of the records costs more (1 M-particle bed 94.5
 // against 98.5 us, 128 scenes of the mix 124 against 131), and served worlds,
 // whose scenes come and go, would capture their graphs anew at each change.
