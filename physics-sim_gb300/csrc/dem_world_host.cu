@@ -1690,13 +1690,10 @@ void World::flip() {
         }                                                                                 \
     } while (0)
 
-// Capture R steps as one graph: per step the LOM kernel, a conditional node
-// whose body is the rebuild (its condition is set on the device by the LOM
-// kernel's last warp or by k_decide), and the Simulation kernel (followed by
-// k_end_step in large worlds).
 // Capture R steps as one graph: the first step's LOM kernel, then per step a
 // conditional node whose body is the rebuild (its condition set on the device
-// by the LOM pass before it) and the Simulation kernel, fused with the next
+// by the LOM pass before it, in large worlds by k_decide or k_end_step) and
+// the Simulation kernel, fused with the next
 // step's LOM pass for all but the last step (with fuse_lom; otherwise every
 // step has its own LOM kernel).  The buffer swaps of the fused
 // steps are applied to the captured launches and undone afterwards: they take
