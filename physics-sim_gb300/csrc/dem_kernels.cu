@@ -134,14 +134,18 @@ struct F3 {
 // (float)(sqrt(dx^2 + dy^2) - (lh + ll)) with the differences, the root and
 // the subtraction in double (lh + ll exact in double), the F64 branch of both
 // distances.  Double precision runs at 1/64 of the float rate here, so the
-// value is first formed in pairs of floats, to 2^-42 of the root (differences
-// and squares exact to a pair, one Newton correction of the float root whose
-// residual is exact), and taken if moving it by that much either way rounds
-// to the same float: the double evaluation, whose own roundings are below
-// 2^-51, then rounds to it too.  Otherwise (one evaluation in ~4,000, or
-// operands outside the range in which the pairs are exact) the expression is
-// evaluated as written.  30,011-particle bed, F64 distances: 13.0 -> 10.0 us a
-// step.
+// value is first formed in pairs of floats, and taken if moving it either way
+// by all that it and the double evaluation can be off together rounds to the
+// same float: the double evaluation then rounds to it too.
+// With u = 2^-24: the pair holds the root to 12.1 u^2 root (differences and
+// squares exact to a pair, one Newton correction of the float root whose
+// residual is exact); the sums with the length, whose terms are up to
+// u (root + lh) each, and moving the value add 5 u^2 root + 4 u^2 lh; the
+// double evaluation's own roundings are below 0.2 u^2 (root + lh).  The room
+// is 5 u^2 (4 root + lh), which grows with the length as well: of two
+// particles that overlap by nearly all of their radii the root is far below lh.
+// Otherwise (or with operands outside the range in which the pairs are exact)
+// the expression is evaluated as written.
 __device__ __forceinline__ float gap_f64(float4 pa, float4 pb, float lh, float ll) {
     const auto two_sum = [](float x, float y, float &err) {  // x + y = sum + err (Knuth)
         const float sum = x + y, yy = sum - x, xx = sum - yy;
@@ -160,7 +164,7 @@ __device__ __forceinline__ float gap_f64(float4 pa, float4 pb, float lh, float l
     const float g0 = two_sum(root, -lh, gl);
     gl = gl + (fix - ll);
     const float g = two_sum(g0, gl, rest);
-    const float err = root * 2.4e-13f;
+    const float err = (4.0f * root + fabsf(lh)) * 1.8e-14f;
     if (root > 1e-9f && root < 1e9f && g + (rest + err) == g && g + (rest - err) == g) return g;
     const double dx = (double)pa.x - (double)pb.x, dy = (double)pa.y - (double)pb.y;
     return (float)(sqrt(dx * dx + dy * dy) - ((double)lh + (double)ll));
