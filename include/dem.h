@@ -177,8 +177,8 @@ typedef struct dem_stats {
                                    ranks beyond 15 in the scan order, or an AABB 31 or more buckets
                                    wide (the bucket grid is much finer than the particles); 4 a large
                                    particle touching more than 2048 particles at once; 8 a step
-                                   kernel's wait for its own blocks ran out of time (reported as
-                                   DEM_E_TIMEOUT by the next call that waits) */
+                                   kernel's wait for its own blocks ran out of time (the calls that
+                                   wait or read state, and every step, then return DEM_E_TIMEOUT) */
     int32_t reserved;
     int64_t kernel_launches;    /* kernels this library launched on the context's stream */
     int64_t list_overflows;     /* particles whose candidates exceeded the list (searched the cells) */

@@ -41,6 +41,11 @@ int dem_debug_kernel_time(dem_ctx *ctx, const char *kernel, double *total_ms, in
 int dem_batch_kernel_timing(dem_batch *b, int32_t enable);
 int dem_batch_kernel_time(dem_batch *b, const char *kernel, double *total_ms, int64_t *launches);
 
+/* The waits between the blocks of the step kernels to come find nothing and
+ * give up after a fraction of a millisecond (at most two seconds otherwise),
+ * which ends the kernel; the context's calls return DEM_E_TIMEOUT from then on. */
+int dem_debug_fail_waits(dem_ctx *ctx);
+
 #ifdef __cplusplus
 }
 #endif

@@ -251,6 +251,11 @@ int dem_debug_kernel_timing(dem_ctx *ctx, int32_t enable) {
     return DEM_OK;
 }
 
+int dem_debug_fail_waits(dem_ctx *ctx) {
+    CTX_GUARD(ctx);
+    return world_rc(ctx, ctx->world.fail_waits());
+}
+
 int dem_debug_kernel_time(dem_ctx *ctx, const char *kernel, double *total_ms, int64_t *launches) {
     CTX_GUARD(ctx);
     if (!kernel) return set_err(ctx, DEM_E_INVALID, "kernel is NULL");

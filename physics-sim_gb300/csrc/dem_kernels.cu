@@ -2497,8 +2497,8 @@ void launch_stage_out(const DevWorld &w, const RefArrays &r, const StageItem *it
 // words, both coalesced
 constexpr int COPY_THREADS = 256;
 __global__ void __launch_bounds__(COPY_THREADS) k_copies(const HostCopy *__restrict__ c, int n,
-                                                          const int32_t *guard) {
-    if (guard && *guard) return;
+                                                          const int32_t *guard, const uint32_t *guard2) {
+    if (guard && (*guard != 0 || *guard2 == 1u)) return;
     __shared__ int s_k;
     const long long b = blockIdx.x;
     if (threadIdx.x == 0) {
@@ -2534,9 +2534,10 @@ __global__ void __launch_bounds__(COPY_THREADS) k_copies(const HostCopy *__restr
     }
 }
 
-void launch_copies(const HostCopy *c, int n, long long pieces, const int32_t *guard, cudaStream_t st) {
+void launch_copies(const HostCopy *c, int n, long long pieces, const int32_t *guard, const uint32_t *guard2,
+                   cudaStream_t st) {
     if (n <= 0 || pieces <= 0) return;
-    k_copies<<<(unsigned)pieces, COPY_THREADS, 0, st>>>(c, n, guard);
+    k_copies<<<(unsigned)pieces, COPY_THREADS, 0, st>>>(c, n, guard, guard2);
 }
 
 // ------------------------------------------------------- Fix / Drop / Release

@@ -29,7 +29,8 @@
 namespace demgb {
 
 // A wait for the other blocks gives up after this many clock cycles (about
-// two seconds; a step takes microseconds), sets device error 8 and ends the run.
+// two seconds; a step takes microseconds), sets device error 8, tells the host
+// and ends the run.
 constexpr long long WAIT_CYCLES = 4000000000LL;
 
 // shared memory of a block of TB threads, in words a thread: 5 fields of 14
@@ -264,6 +265,7 @@ __device__ __forceinline__ uint32_t wait_for(const uint32_t *p, uint32_t mask, u
     } while (clock64() - t0 < WAIT_CYCLES && ld_relaxed(&R.fail) == 0u);
     atomicOr(err, 8);
     st_relaxed(&R.fail, 1u);
+    *(volatile int32_t *)&R.report->failed = 1;
     return WAIT_FAILED;
 }
 
@@ -384,7 +386,9 @@ struct Run {
 
     // After `done` steps: meet the other blocks.  Breaks are applied by block 0
     // while the others wait once more (R.gen); the end of the run needs no
-    // wait, nothing that block 0 writes then is read again.  If a particle
+    // wait, nothing that block 0 writes then is read again.  A block whose wait
+    // for R.gen gave up goes on to the next barrier: the run has failed, and
+    // the host hands out none of its state.  If a particle
     // left its list and this rebuild need not reorder the particles, lists(done)
     // rebuilds them (false: a wait failed).  True when the run ends.
     template <class Lists>
@@ -430,7 +434,7 @@ __global__ void __launch_bounds__(TB, 1) k_steps(DevWorld w, cudaGraphConditiona
     __shared__ uint32_t s_any[3];
     StepRun &R = *w.run;
     const int todo = R.todo;
-    const bool lom_done = R.lom_done != 0, failed = R.fail != 0;
+    const bool lom_done = R.lom_done != 0, failed = R.fail == 1u;
     float *rec_out = R.rec_out == nullptr ? nullptr : R.rec_out + (long long)R.rec_per * R.done;
     const int rec_per = R.rec_per;
     if (failed || todo <= 0) {  // uniform over the grid: no block changes these before all have read them
@@ -682,7 +686,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 1) k_sweep(DevWorld w, cudaGrap
     __shared__ uint32_t s_any[3];
     StepRun &R = *w.run;
     const int todo = R.todo;
-    const bool lom_done = R.lom_done != 0, failed = R.fail != 0;
+    const bool lom_done = R.lom_done != 0, failed = R.fail == 1u;
     if (failed || todo <= 0) {  // uniform over the grid, as in k_steps
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             cudaGraphSetConditional(more, 0u);

@@ -127,16 +127,23 @@ struct StepRun {
     int32_t lom_done;        // 1: the next step's LOM pass has run
     uint32_t arrive[3];      // barrier counters, used in turn
     uint32_t gen;            // the launch's last barrier whose breaks have been applied
-    uint32_t fail;           // a wait gave up: no run starts any more
+    uint32_t fail;           // 1: a wait gave up, no run starts any more; 2: the next wait does (tests)
     uint32_t links;          // rebuilds by cell chains so far (a chain's number is never 0)
     int32_t linked;          // 1: the lists come from such a rebuild, and cell_start and sorted are of an earlier one
     int32_t rec_scene, rec_base, rec_per;  // recorded scene, its first particle, floats a step
     const int32_t *rec_rows; // [particles of the scene] row of each recorded one, -1 the others; null: none
     float *rec_out;
+    uint32_t skew;           // the barrier counters' start, 0; else no barrier is ever complete (tests)
+    struct RunReport *report;
+};
+// What the host learns of the runs without a copy: words in page-locked host
+// memory that the device writes, read after the stream has been waited for.
+struct RunReport {
+    int32_t failed;  // a wait gave up: the world's state is of no step
 };
 // before every launch of the kernel
 __device__ __forceinline__ void clear_run_barrier(StepRun &R) {
-    R.arrive[0] = R.arrive[1] = R.arrive[2] = 0u;
+    R.arrive[0] = R.arrive[1] = R.arrive[2] = R.skew;
     R.gen = 0u;
 }
 
@@ -368,8 +375,9 @@ struct HostCopy {
     long long piece0;
 };
 // every piece of copies c[0..n) (`pieces` in all); nothing if guard != NULL
-// and *guard != 0
-void launch_copies(const HostCopy *c, int n, long long pieces, const int32_t *guard, cudaStream_t st);
+// and *guard != 0 or *guard2 == 1 (StepRun::fail)
+void launch_copies(const HostCopy *c, int n, long long pieces, const int32_t *guard, const uint32_t *guard2,
+                   cudaStream_t st);
 
 // Fix / Drop / Release events (src/shaders/event_handling/{Fix,Drop,Release}.wgsl)
 // on `count` particles of the scene whose first particle is `base`, given

@@ -78,6 +78,7 @@ World::~World() {
     release();
     if (ref_block) cudaFree(ref_block);
     if (pin) cudaFreeHost(pin);
+    if (report) cudaFreeHost(report);
     if (d_items) cudaFree(d_items);
     if (d_copies) cudaFree(d_copies);
     for (auto e : xfer_ev) cudaEventDestroy(e);
@@ -525,6 +526,9 @@ int World::alloc(int N, int C, int B, int S, int M, int MP, int TB, uint32_t ev_
     w.big_acc = dalloc<int32_t>(owned, 16 * (size_t)std::max(TB, 1), ok);
     w.big_scene = dalloc<int32_t>(owned, std::max(TB, 1), ok);
     w.run = dalloc<StepRun>(owned, 1, ok);
+    if (!report && cudaHostAlloc(reinterpret_cast<void **>(&report), sizeof(RunReport), cudaHostAllocMapped) != cudaSuccess)
+        report = nullptr, ok = false;
+    if (report) *report = RunReport{};
     run_block = steps_block(N);
     w.cell_head = dalloc<unsigned long long>(owned, run_block ? (size_t)C : 1, ok);
     w.cell_next = dalloc<int32_t>(owned, run_block ? (size_t)N : 1, ok);
@@ -544,7 +548,9 @@ int World::alloc(int N, int C, int B, int S, int M, int MP, int TB, uint32_t ev_
     CK(cudaMemsetAsync(w.tickets, 0, 2 * sizeof(uint32_t), stream));
     CK(cudaMemsetAsync(w.nl, 0, sizeof(int4) * 2 * (size_t)(N > 0 ? N : 1), stream));
     CK(cudaMemsetAsync(w.err, 0, sizeof(int32_t), stream));
-    CK(cudaMemsetAsync(w.run, 0, sizeof(StepRun), stream));
+    StepRun run{};
+    run.report = report;
+    CK(cudaMemcpyAsync(w.run, &run, sizeof run, cudaMemcpyHostToDevice, stream));
     if (run_block) CK(cudaMemsetAsync(w.cell_head, 0, 8 * (size_t)C, stream));
     {
         static const int32_t one = 1;  // the first rebuild reorders
@@ -976,7 +982,7 @@ int World::stage_many(const int32_t *idx, const dem_scene *const *scs, int count
         if (nc > 0) {
             ce = cudaMemcpyAsync(d_copies, hc, sizeof(HostCopy) * nc, cudaMemcpyHostToDevice, stream);
             if (ce == cudaSuccess) {
-                launch_copies(d_copies, nc, pieces, nullptr, stream);
+                launch_copies(d_copies, nc, pieces, nullptr, nullptr, stream);
                 ce = cudaGetLastError();
             }
         }
@@ -1943,7 +1949,8 @@ int World::refresh_graphs() {
 
 int World::step(int n_steps) {
     if (n_steps < 0) return fail(DEM_E_INVALID, "n_steps < 0");
-    const int rc = refresh_graphs();
+    int rc = runs_intact();
+    if (rc == DEM_OK) rc = refresh_graphs();
     if (rc) return rc;
     if (n_steps > 0 && runs_resident()) return run_steps(n_steps, RunRecord{});
     int k = 0;
@@ -1982,11 +1989,29 @@ int World::step(int n_steps) {
     return DEM_OK;
 }
 
+// After a wait that gave up the state is of no step and nothing steps any
+// more: the calls that wait for the stream and those that step say so.  The
+// device has set the word by the time a wait for the stream returns.
+int World::runs_intact() {
+    if (!report || *(volatile int32_t *)&report->failed == 0) return DEM_OK;
+    return fail(DEM_E_TIMEOUT, "a wait between the blocks of a step kernel gave up; create the world anew");
+}
+
+// debug: no barrier of the runs to come completes, and the waits give up soon
+int World::fail_waits() {
+    const uint32_t next = 2u, skew = 512u;  // 512: never the number of blocks (at most one an SM)
+    CK(cudaMemcpyAsync(&d.run->fail, &next, sizeof next, cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(&d.run->skew, &skew, sizeof skew, cudaMemcpyHostToDevice, stream));
+    CK(cudaStreamSynchronize(stream));
+    return DEM_OK;
+}
+
 int World::sync() {
     CK(cudaStreamSynchronize(stream));
+    const int rc = runs_intact();
+    if (rc) return rc;
     int32_t e = 0;
     CK(cudaMemcpy(&e, d.err, 4, cudaMemcpyDeviceToHost));
-    if (e & 8) return fail(DEM_E_TIMEOUT, "a wait between the blocks of a step kernel gave up");
     if (e) return fail(DEM_E_STATE, "device error flags set: " + std::to_string(e));
     return DEM_OK;
 }
@@ -2104,6 +2129,8 @@ int World::download_many(const int32_t *idx, dem_scene *const *outs, int count) 
         out->grid = h.grid;
     };
     auto first_error = [&]() -> int {
+        const int r1 = runs_intact();
+        if (r1) return r1;
         for (int i = 0; i < nt; ++i)
             if (h_err[i]) {
                 const int r2 = unstage_error(h_err[i]);
@@ -2132,7 +2159,7 @@ int World::download_many(const int32_t *idx, dem_scene *const *outs, int count) 
         }
         if (nc > 0) {
             CK(cudaMemcpyAsync(d_copies, hc, sizeof(HostCopy) * nc, cudaMemcpyHostToDevice, stream));
-            launch_copies(d_copies, nc, pieces, d_item_err + nt, stream);
+            launch_copies(d_copies, nc, pieces, d_item_err + nt, &d.run->fail, stream);
             CK(cudaGetLastError());
         }
         cudaError_t ce = fetch_bonds();
@@ -2242,6 +2269,8 @@ int World::set_properties(int s, int32_t *selections, const int32_t *props) {
     cudaFree(dout);
     cudaFree(dprops);
     if (e != cudaSuccess || e2 != cudaSuccess) return fail(DEM_E_CUDA, "set_properties failed");
+    const int rc = runs_intact();
+    if (rc) return rc;
     for (int i = 0; i < n; ++i)
         if (selections[i] != 0 && props[9] == 1) h.r_max = std::max(h.r_max, f[23]);
     if (any && (props[0] == 1 || props[1] == 1 || props[9] == 1)) return force_rebuild(false);
@@ -2287,7 +2316,7 @@ int World::fixity_event(int s, int kind, int32_t *selections, int throw_vel, flo
     const cudaError_t e = cudaStreamSynchronize(stream);
     cudaFree(dbuf);
     if (e != cudaSuccess) return fail(DEM_E_CUDA, std::string("fixity event: ") + cudaGetErrorString(e));
-    return DEM_OK;
+    return runs_intact();
 }
 
 // State::get_datum (state.rs:708-737): means over the selected particles of
@@ -2314,6 +2343,8 @@ int World::get_datum(int s, const int32_t *selections, double out[10]) {
     const cudaError_t e = cudaStreamSynchronize(stream);
     cudaFree(dbuf);
     if (e != cudaSuccess) return fail(DEM_E_CUDA, std::string("datum: ") + cudaGetErrorString(e));
+    const int rc = runs_intact();
+    if (rc) return rc;
     double sums[10] = {0.0};
     for (int t = 0; t < k; ++t) {
         const float *g = &f[10 * (size_t)t];
@@ -2379,7 +2410,8 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
     for (int s0 = 0; rc == DEM_OK && s0 < n_steps; s0 += chunk) {
         const int m = std::min(chunk, n_steps - s0);
         if (d_sel) {
-            rc = refresh_graphs();
+            rc = runs_intact();
+            if (rc == DEM_OK) rc = refresh_graphs();
             if (rc == DEM_OK) rc = run_steps(m, RunRecord{d_sel, s, h.particle_base, (int)per, d_rows});
         }
         for (int j = 0; j < m && rc == DEM_OK && !d_sel; ++j) {
@@ -2393,6 +2425,7 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
             rc = fail(DEM_E_CUDA, std::string("record: ") + cudaGetErrorString(e));
             break;
         }
+        if ((rc = runs_intact()) != DEM_OK) break;  // the rows were not written
         for (int j = 0; j < m; ++j) {
             double sums[10] = {0.0};
             for (int t = 0; t < k; ++t) {
@@ -2410,6 +2443,8 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
 
 int World::drain_events(std::vector<dem_break_event> &out) {
     CK(cudaStreamSynchronize(stream));
+    const int rc = runs_intact();
+    if (rc) return rc;
     unsigned long long cnt = 0;
     CK(cudaMemcpy(&cnt, d.ev_count, sizeof cnt, cudaMemcpyDeviceToHost));
     size_t k = (size_t)std::min<unsigned long long>(cnt, d.ev_cap);

@@ -135,6 +135,7 @@ class World {
     void rec_event(int kind, cudaStream_t st);
     int kernel_time(int kind, double *ms, long long *n);
     void set_timing(bool on);
+    int fail_waits();  // debug
 
   private:
     int fail(int code, const std::string &msg);
@@ -164,6 +165,8 @@ class World {
     bool runs_resident() const;
     int run_steps(int n_steps, const RunRecord &rec);
     int refresh_graphs();
+    RunReport *report = nullptr;   // page-locked (StepRun::report)
+    int runs_intact();
     bool was_resident = false;
     void drop_graph();
     bool dense_cells() const;

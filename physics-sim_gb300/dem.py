@@ -134,7 +134,7 @@ SYMBOLS = ["dem_abi_version", "dem_ext_defaults", "dem_last_error", "dem_grid_ca
            "dem_generate_bonds", "dem_bondgen_last_error", "dem_event", "dem_get_datum",
            "dem_batch_event", "dem_batch_get_datum", "dem_batch_upload_many", "dem_batch_download_many",
            "dem_record", "dem_batch_record",
-           "dem_server_cancel"]
+           "dem_server_cancel", "dem_debug_fail_waits"]
 
 _lib = None
 
@@ -179,6 +179,7 @@ def lib(path=None):
     L.dem_debug_broad_phase.argtypes = [C.c_void_p, _IP, _IP, _IP, C.POINTER(C.c_int32)]
     L.dem_debug_search_grid.argtypes = [C.c_void_p, _FP, _FP, _FP, _IP, _IP]
     L.dem_debug_kernel_timing.argtypes = [C.c_void_p, C.c_int32]
+    L.dem_debug_fail_waits.argtypes = [C.c_void_p]
     L.dem_debug_kernel_time.argtypes = [C.c_void_p, C.c_char_p, C.POINTER(C.c_double),
                                         C.POINTER(C.c_int64)]
     L.dem_broad_phase_noalloc.argtypes = [C.c_void_p, C.c_int32, C.c_float, C.c_float, C.c_float,
@@ -500,6 +501,11 @@ class Context:
 
     def stream(self):
         return lib().dem_stream(self.h)
+
+    def fail_waits(self):
+        """dem_debug_fail_waits: the waits between a step kernel's blocks give up."""
+        L = lib()
+        _check(L, self.h, L.dem_debug_fail_waits(self.h))
 
     def kernel_timing(self, on):
         L = lib()
