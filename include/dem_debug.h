@@ -41,6 +41,16 @@ int dem_debug_kernel_time(dem_ctx *ctx, const char *kernel, double *total_ms, in
 int dem_batch_kernel_timing(dem_batch *b, int32_t enable);
 int dem_batch_kernel_time(dem_batch *b, const char *kernel, double *total_ms, int64_t *launches);
 
+/* Runs: a step call of a small world is one kernel (a run), where the library
+ * finds it faster; results do not depend on it.  dem_debug_runs chooses: 0 the
+ * library's choice, 1 a launch a step, 2 as if the device refused every run
+ * (which also ends in launches).  dem_debug_run_calls: the step calls, and
+ * chunks of dem_record, that were runs so far. */
+int dem_debug_runs(dem_ctx *ctx, int32_t mode);
+int64_t dem_debug_run_calls(dem_ctx *ctx);
+/* The same for a batch. */
+int dem_batch_runs(dem_batch *b, int32_t mode);
+int64_t dem_batch_run_calls(dem_batch *b);
 /* The waits between the blocks of the step kernels to come find nothing and
  * give up after a fraction of a millisecond (at most two seconds otherwise),
  * which ends the kernel; the context's calls return DEM_E_TIMEOUT from then on. */

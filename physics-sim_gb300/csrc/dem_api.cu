@@ -251,6 +251,13 @@ int dem_debug_kernel_timing(dem_ctx *ctx, int32_t enable) {
     return DEM_OK;
 }
 
+int dem_debug_runs(dem_ctx *ctx, int32_t mode) {
+    CTX_GUARD(ctx);
+    return world_rc(ctx, ctx->world.set_runs(mode));
+}
+
+int64_t dem_debug_run_calls(dem_ctx *ctx) { return ctx ? ctx->world.run_calls : 0; }
+
 int dem_debug_fail_waits(dem_ctx *ctx) {
     CTX_GUARD(ctx);
     return world_rc(ctx, ctx->world.fail_waits());

@@ -178,6 +178,14 @@ int dem_batch_kernel_timing(dem_batch *b, int32_t enable) {
     return DEM_OK;
 }
 
+int dem_batch_runs(dem_batch *b, int32_t mode) {
+    BATCH_GUARD(b);
+    const int rc = b->world.set_runs(mode);
+    return rc ? bset(b, rc, b->world.err.c_str()) : DEM_OK;
+}
+
+int64_t dem_batch_run_calls(dem_batch *b) { return b ? b->world.run_calls : 0; }
+
 int dem_batch_kernel_time(dem_batch *b, const char *kernel, double *total_ms, int64_t *launches) {
     BATCH_GUARD(b);
     if (!kernel) return bset(b, DEM_E_INVALID, "kernel is NULL");

@@ -112,6 +112,10 @@ cudaError_t launch_steps(const DevWorld &w, int block, cudaStream_t st, cudaGrap
     const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void *>(fn),
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
+    int per = 0;
+    const cudaError_t o = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, block, (size_t)bytes);
+    if (o != cudaSuccess) return o;
+    if ((long long)per * device_sms() < grid) return cudaErrorCooperativeLaunchTooLarge;
     c.gridDim = dim3((unsigned)grid);
     c.blockDim = dim3((unsigned)block);
     c.dynamicSmemBytes = (size_t)bytes;

@@ -1812,7 +1812,7 @@ int World::capture_run(cudaGraphExec_t *out) {
         e = cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
         cudaGraph_t done = nullptr;
-        e = launch_steps(d, run_block, side, more, due, kernel_form, &par_pv, par_ps);
+        e = runs_fault ? cudaErrorCooperativeLaunchTooLarge : launch_steps(d, run_block, side, more, due, kernel_form, &par_pv, par_ps);
         const cudaGraphNode_t *deps = nullptr;
         size_t ndeps = 0;
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1845,20 +1845,44 @@ int World::capture_run(cudaGraphExec_t *out) {
 // a step: 128 bonded particles 19.4 -> 4.2, 4,096 falling 13.8 -> 2.7, 16,384
 // bonded 18.2 -> 5.7, a 30,011-particle bed with F64 distances 35.9 -> 9.8, a
 // 262,144-particle bed 44.3 -> 31.4); k_big_narrow is a launch of its own.
-bool World::runs_resident() const { return use_graphs && !timing && !has_bigs && run_block > 0; }
+bool World::runs_resident() const {
+    return use_graphs && !timing && !has_bigs && run_block > 0 && !runs_refused && !runs_off;
+}
 
-// one run of n_steps, recording the datum of the particles in rec.rows
-int World::run_steps(int n_steps, const RunRecord &rec) {
+// Whether the graph of a run is there or could be captured.  Where the device
+// does not take it (a cooperative grid beyond what a partitioned or shared
+// device holds at once), the world steps by launches from then on.
+bool World::ready_run() {
     const int p = parity;
-    if (!graph_run[p]) {
-        const int rc = capture_run(&graph_run[p]);
-        if (rc) return rc;
-    }
+    if (graph_run[p] || capture_run(&graph_run[p]) == DEM_OK) return true;
+    cudaGetLastError();
+    err.clear();
+    runs_refused = true;
+    return false;
+}
+
+// One run of n_steps, recording the datum of the particles in rec.rows; false,
+// with no step taken, when the device refuses it.
+bool World::run_steps(int n_steps, const RunRecord &rec) {
+    if (!ready_run()) return false;
     launch_run_begin(d, n_steps, rec, stream);
-    CK(cudaGetLastError());
-    CK(cudaGraphLaunch(graph_run[p], stream));
+    if (cudaGetLastError() != cudaSuccess || cudaGraphLaunch(graph_run[parity], stream) != cudaSuccess) {
+        cudaGetLastError();
+        runs_refused = true;
+        return false;
+    }
+    ++run_calls;
     launches += 2;
     host_step += n_steps;
+    return true;
+}
+
+int World::set_runs(int mode) {
+    if (mode < 0 || mode > 2) return fail(DEM_E_INVALID, "runs mode out of range");
+    runs_off = mode == 1;
+    runs_fault = mode == 2;
+    runs_refused = false;
+    drop_graph();
     return DEM_OK;
 }
 
@@ -1952,7 +1976,11 @@ int World::step(int n_steps) {
     int rc = runs_intact();
     if (rc == DEM_OK) rc = refresh_graphs();
     if (rc) return rc;
-    if (n_steps > 0 && runs_resident()) return run_steps(n_steps, RunRecord{});
+    if (n_steps > 0 && runs_resident()) {
+        if (run_steps(n_steps, RunRecord{})) return DEM_OK;
+        rc = refresh_graphs();
+        if (rc) return rc;
+    }
     int k = 0;
     if (use_graphs && !timing && n_steps > 0) {
         while (n_steps - k >= graph_steps) {
@@ -2391,7 +2419,10 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
     const int chunk = (int)std::max<long long>(1, std::min<long long>(n_steps, (1LL << 24) / per));
     // a resident run records inside its kernel, which looks up each particle's
     // row; else a gather after every step takes the list of recorded particles
-    const bool resident = runs_resident() && run_block != SWEEP_THREADS;
+    int rc = runs_intact();
+    if (rc == DEM_OK) rc = refresh_graphs();
+    if (rc) return rc;
+    const bool resident = runs_resident() && run_block != SWEEP_THREADS && ready_run();
     std::vector<int32_t> row_of;
     if (resident) {
         row_of.assign((size_t)h.n, -1);
@@ -2404,15 +2435,17 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
     const int32_t *d_sel = resident ? d_idx : nullptr;
     float *d_rows = reinterpret_cast<float *>(d_idx + idx.size());
     std::vector<float> f((size_t)(per * chunk));
-    int rc = DEM_OK;
     cudaError_t e = cudaMemcpyAsync(d_idx, idx.data(), sizeof(int32_t) * idx.size(), cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) rc = fail(DEM_E_CUDA, std::string("record: ") + cudaGetErrorString(e));
     for (int s0 = 0; rc == DEM_OK && s0 < n_steps; s0 += chunk) {
         const int m = std::min(chunk, n_steps - s0);
         if (d_sel) {
             rc = runs_intact();
-            if (rc == DEM_OK) rc = refresh_graphs();
-            if (rc == DEM_OK) rc = run_steps(m, RunRecord{d_sel, s, h.particle_base, (int)per, d_rows});
+            if (rc == DEM_OK && !run_steps(m, RunRecord{d_sel, s, h.particle_base, (int)per, d_rows})) {
+                cudaStreamSynchronize(stream);  // the rest by launches
+                cudaFree(dbuf);
+                return record(s, selections, n_steps - s0, rows + 10LL * s0);
+            }
         }
         for (int j = 0; j < m && rc == DEM_OK && !d_sel; ++j) {
             rc = step(1);

@@ -136,6 +136,8 @@ class World {
     int kernel_time(int kind, double *ms, long long *n);
     void set_timing(bool on);
     int fail_waits();  // debug
+    long long run_calls = 0;       // step calls (and chunks of a record) taken as runs
+    int set_runs(int mode);        // debug: 0 the library's choice, 1 launches, 2 every run refused
 
   private:
     int fail(int code, const std::string &msg);
@@ -163,7 +165,10 @@ class World {
     cudaGraphExec_t graph_run[2] = {nullptr, nullptr};  // a run of steps, per buffer parity
     int capture_run(cudaGraphExec_t *out);
     bool runs_resident() const;
-    int run_steps(int n_steps, const RunRecord &rec);
+    bool runs_refused = false;     // a run could not be captured or launched: launches from then on
+    bool runs_off = false, runs_fault = false;  // debug (set_runs)
+    bool ready_run();
+    bool run_steps(int n_steps, const RunRecord &rec);
     int refresh_graphs();
     RunReport *report = nullptr;   // page-locked (StepRun::report)
     int runs_intact();

@@ -134,7 +134,8 @@ SYMBOLS = ["dem_abi_version", "dem_ext_defaults", "dem_last_error", "dem_grid_ca
            "dem_generate_bonds", "dem_bondgen_last_error", "dem_event", "dem_get_datum",
            "dem_batch_event", "dem_batch_get_datum", "dem_batch_upload_many", "dem_batch_download_many",
            "dem_record", "dem_batch_record",
-           "dem_server_cancel", "dem_debug_fail_waits"]
+           "dem_server_cancel", "dem_debug_fail_waits", "dem_debug_runs", "dem_debug_run_calls",
+           "dem_batch_runs", "dem_batch_run_calls"]
 
 _lib = None
 
@@ -180,6 +181,8 @@ def lib(path=None):
     L.dem_debug_search_grid.argtypes = [C.c_void_p, _FP, _FP, _FP, _IP, _IP]
     L.dem_debug_kernel_timing.argtypes = [C.c_void_p, C.c_int32]
     L.dem_debug_fail_waits.argtypes = [C.c_void_p]
+    L.dem_debug_runs.argtypes = L.dem_batch_runs.argtypes = [C.c_void_p, C.c_int32]
+    L.dem_debug_run_calls.argtypes = L.dem_batch_run_calls.argtypes = [C.c_void_p]
     L.dem_debug_kernel_time.argtypes = [C.c_void_p, C.c_char_p, C.POINTER(C.c_double),
                                         C.POINTER(C.c_int64)]
     L.dem_broad_phase_noalloc.argtypes = [C.c_void_p, C.c_int32, C.c_float, C.c_float, C.c_float,
@@ -246,6 +249,7 @@ def lib(path=None):
                         "dem_server_destroy", "dem_server_last_error", "dem_server_stream",
                         "dem_tune_last_error", "dem_bondgen_last_error"):
             getattr(L, name).restype = C.c_int
+    L.dem_debug_run_calls.restype = L.dem_batch_run_calls.restype = C.c_int64
     _lib = L
     return L
 
@@ -507,6 +511,15 @@ class Context:
         L = lib()
         _check(L, self.h, L.dem_debug_fail_waits(self.h))
 
+    def runs(self, mode):
+        """dem_debug_runs: 0 the library's choice, 1 a launch a step, 2 every run refused."""
+        L = lib()
+        _check(L, self.h, L.dem_debug_runs(self.h, int(mode)))
+
+    def run_calls(self):
+        """dem_debug_run_calls: step calls taken as one kernel so far."""
+        return int(lib().dem_debug_run_calls(self.h))
+
     def kernel_timing(self, on):
         L = lib()
         _check(L, self.h, L.dem_debug_kernel_timing(self.h, 1 if on else 0))
@@ -701,6 +714,14 @@ class Batch:
         self._check(lib().dem_batch_download_many(self.h, t.n, C.c_void_p(t.idx.ctypes.data),
                                                   C.c_void_p(t.ptrs.ctypes.data)))
         t.read_control()
+
+    def runs(self, mode):
+        """dem_batch_runs: 0 the library's choice, 1 a launch a step, 2 every run refused."""
+        self._check(lib().dem_batch_runs(self.h, int(mode)))
+
+    def run_calls(self):
+        """dem_batch_run_calls: step calls taken as one kernel so far."""
+        return int(lib().dem_batch_run_calls(self.h))
 
     def kernel_timing(self, on):
         """CUDA-event timing of every kernel kind (plain launches while on)."""
