@@ -1945,24 +1945,42 @@ void World::update_split() {
     drop_graph();
 }
 
+// Whether a call of n_steps steps is a run.  A call of one step is a launch a
+// step while the cell table is as new as the lists: the kernels of a run load
+// and store the whole state for it (step and wait, microseconds by launches
+// and by runs: 128 particles 38 / 41, 16,384 42 / 46, 100,000 49 / 57, 262,144
+// 62 / 70; a batch of 64 scenes 52 / 63), two steps are faster as a run (65 /
+// 47, 70 / 53, 84 / 74, 106 / 102).  After a run the first launch costs a
+// rebuild (~100 us), so single steps stay runs until SINGLES of them came in a row.
+constexpr int SINGLES = 32;
+bool World::take_run(int n_steps) {
+    if (!runs_resident()) return false;
+    if (n_steps != 1) {
+        singles = 0;
+        return true;
+    }
+    return was_resident && ++singles < SINGLES;
+}
+
 // what the captured graphs depend on, brought up to date before a call steps
-int World::refresh_graphs() {
+// (run: as a run)
+int World::refresh_graphs(bool run) {
     update_param_source();
     update_split();
-    const bool resident = runs_resident();
     // the records of a world that runs resident sit in L2 wherever they are:
     // its rebuilds stay within the run, all but one in 32
-    const int every = reorder_every > 0 ? reorder_every : resident ? 32 : (sh.size() == 1 ? 3 : 8);
+    const int every = reorder_every > 0 ? reorder_every : runs_resident() ? 32 : (sh.size() == 1 ? 3 : 8);
     if (every != d.reorder_every) {
         d.reorder_every = every;
         drop_graph();
     }
-    if (was_resident && !resident) {
+    if (was_resident && !run) {
         // the cell table may be of an earlier rebuild than the lists
         const int rc = force_rebuild(false);
         if (rc) return rc;
     }
-    was_resident = resident;
+    was_resident = run;
+    singles = run ? singles : 0;
     if (par_ps != graph_ps || std::memcmp(&par_pv, &graph_par, sizeof(ScenePar)) != 0) {
         drop_graph();
         graph_ps = par_ps;
@@ -1974,11 +1992,13 @@ int World::refresh_graphs() {
 int World::step(int n_steps) {
     if (n_steps < 0) return fail(DEM_E_INVALID, "n_steps < 0");
     int rc = runs_intact();
-    if (rc == DEM_OK) rc = refresh_graphs();
+    if (rc || n_steps == 0) return rc;
+    const bool run = take_run(n_steps);
+    rc = refresh_graphs(run);
     if (rc) return rc;
-    if (n_steps > 0 && runs_resident()) {
+    if (run) {
         if (run_steps(n_steps, RunRecord{})) return DEM_OK;
-        rc = refresh_graphs();
+        rc = refresh_graphs(false);
         if (rc) return rc;
     }
     int k = 0;
@@ -2408,21 +2428,18 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
     for (int i = 0; i < h.n; ++i)
         if (selections[i] != 0) idx.push_back(i);
     const int k = (int)idx.size();
-    if (k == 0) {
-        for (int j = 0; j < n_steps; ++j) {
-            const int rc = step(1);
-            if (rc) return rc;
-        }
-        return 0;
-    }
+    if (k == 0) return step(n_steps);
     const long long per = 10LL * k;  // floats per recorded step
     const int chunk = (int)std::max<long long>(1, std::min<long long>(n_steps, (1LL << 24) / per));
     // a resident run records inside its kernel, which looks up each particle's
     // row; else a gather after every step takes the list of recorded particles
     int rc = runs_intact();
-    if (rc == DEM_OK) rc = refresh_graphs();
+    bool resident = runs_resident() && run_block != SWEEP_THREADS;
+    // a launch a step from the first on, where it is not in the run: step() per row
+    if (!resident && n_steps >= 16) singles = SINGLES;
+    if (rc == DEM_OK && resident) rc = refresh_graphs(true);
     if (rc) return rc;
-    const bool resident = runs_resident() && run_block != SWEEP_THREADS && ready_run();
+    resident = resident && ready_run();
     std::vector<int32_t> row_of;
     if (resident) {
         row_of.assign((size_t)h.n, -1);

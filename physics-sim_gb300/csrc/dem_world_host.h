@@ -169,7 +169,9 @@ class World {
     bool runs_off = false, runs_fault = false;  // debug (set_runs)
     bool ready_run();
     bool run_steps(int n_steps, const RunRecord &rec);
-    int refresh_graphs();
+    int refresh_graphs(bool run);
+    bool take_run(int n_steps);
+    int singles = 0;               // step calls of one step in a row, while they are runs
     RunReport *report = nullptr;   // page-locked (StepRun::report)
     int runs_intact();
     bool was_resident = false;

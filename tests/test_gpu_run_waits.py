@@ -59,7 +59,7 @@ def test_the_first_call_that_waits_reports_it(n, first):
     sel = np.ones(n, np.int32)
     with dem.Context(copy_scene(sc), p, **ext) as ctx:
         ctx.fail_waits()
-        if first != "record":
+        if first != "record" or n > 77824:  # a sweep records nothing: its record is no run
             ctx.step(3)
         refused({"synchronize": ctx.synchronize, "record": lambda: ctx.record(3, sel),
                  "datum": lambda: ctx.datum(sel), "break_events": ctx.break_events}[first])
