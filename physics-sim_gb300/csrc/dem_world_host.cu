@@ -72,7 +72,36 @@ void RangeAlloc::release(long long off, long long n) {
     }
 }
 
+// Particles of the worlds whose step calls no call has waited for, by device:
+// what the runs of other worlds would share the device with.  A host that
+// only ever waits for a world's stream by itself leaves the world counted.
+constexpr int DEVICES = 64;
+static std::atomic<long long> queued_particles[DEVICES];
+
+long long World::queued_on(int device) {
+    return device >= 0 && device < DEVICES ? queued_particles[device].load(std::memory_order_relaxed) : 0;
+}
+
+void World::count_queued() {
+    if (queued || device < 0 || device >= DEVICES) return;
+    queued = d.N;
+    queued_particles[device].fetch_add(queued, std::memory_order_relaxed);
+}
+
+void World::settled() {
+    if (!queued) return;
+    queued_particles[device].fetch_sub(queued, std::memory_order_relaxed);
+    queued = 0;
+}
+
+cudaError_t World::wait() {
+    const cudaError_t e = cudaStreamSynchronize(stream);
+    settled();
+    return e;
+}
+
 World::~World() {
+    settled();
     set_timing(true);
     set_timing(false);
     release();
@@ -436,7 +465,7 @@ int World::update_live() {
             live[c] = 1;
     }
     CK(cudaMemcpyAsync(live_d, live.data(), chunks, cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     return DEM_OK;
 }
 
@@ -561,7 +590,7 @@ int World::alloc(int N, int C, int B, int S, int M, int MP, int TB, uint32_t ev_
     CK(cudaMemsetAsync(w.cc3, 0, sizeof(int32_t) * (size_t)S, stream));
     CK(cudaMemsetAsync(w.act, 0, sizeof(int32_t) * (size_t)S, stream));
     CK(cudaMemcpyAsync(w.step, &host_step, sizeof(long long), cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     return DEM_OK;
 }
 
@@ -860,7 +889,7 @@ int World::push_det() {
     for (size_t s = 0; s < sh.size(); ++s)
         det[s] = detect_at(sh[s].params.collision_interval, sh[s].cc1_0, host_step - sh[s].step0) ? 1 : 0;
     CK(cudaMemcpyAsync(d.det, det.data(), det.size() * 4, cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     return DEM_OK;
 }
 
@@ -873,7 +902,7 @@ int World::force_rebuild(bool reorder) {
     static const int32_t one = 1;
     CK(cudaMemcpyAsync(d.rebuild, &one, 4, cudaMemcpyHostToDevice, stream));
     if (reorder) CK(cudaMemcpyAsync(d.reorder, &one, 4, cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     return DEM_OK;
 }
 
@@ -884,7 +913,7 @@ int World::push_bigs(int s, int scene_or_free) {
     if (h.big_cap <= 0) return DEM_OK;
     std::vector<int32_t> v(h.big_cap, scene_or_free);
     CK(cudaMemcpyAsync(d.big_scene + h.big_base, v.data(), 4 * (size_t)h.big_cap, cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     update_has_bigs();
     return DEM_OK;
 }
@@ -912,7 +941,7 @@ int World::push_active(int s, bool on, long long steps) {
     long long r = steps;
     CK(cudaMemcpyAsync(d.act + s, &a, 4, cudaMemcpyHostToDevice, stream));
     CK(cudaMemcpyAsync(d.remaining + s, &r, 8, cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     sh[s].active = on;
     return DEM_OK;
 }
@@ -988,7 +1017,7 @@ int World::stage_many(const int32_t *idx, const dem_scene *const *scs, int count
         }
         rc = layouts ? layouts() : DEM_OK;
         if (rc != DEM_OK || ce != cudaSuccess) {
-            cudaStreamSynchronize(stream);  // the tables in the page-locked block are in use until then
+            wait();  // the tables in the page-locked block are in use until then
             return ce != cudaSuccess ? fail(DEM_E_CUDA, cudaGetErrorString(ce)) : rc;
         }
     } else {
@@ -1048,7 +1077,7 @@ int World::stage_many(const int32_t *idx, const dem_scene *const *scs, int count
     {
         // waited for even after a failed call: until then the copies may be
         // reading the callers' arrays
-        const cudaError_t se = cudaStreamSynchronize(stream);
+        const cudaError_t se = wait();
         if (ce == cudaSuccess) ce = se;
     }
     if (ce != cudaSuccess) return fail(DEM_E_CUDA, cudaGetErrorString(ce));
@@ -1090,7 +1119,7 @@ int World::stage_many(const int32_t *idx, const dem_scene *const *scs, int count
     CK(send(d.mats, h_mats, sizeof(Mat), rm));
     CK(send(d.pair, h_pair, 8, rp));
     CK(send(d.par, h_par, sizeof(ScenePar), rs));
-    CK(cudaStreamSynchronize(stream));  // the page-locked block is reused by the next transfer
+    CK(wait());  // the page-locked block is reused by the next transfer
     return DEM_OK;
 }
 
@@ -1103,7 +1132,7 @@ int World::push_materials(int s) {
     CK(cudaMemcpyAsync(d.mats + h.mat_base, mats.data(), M * sizeof(Mat), cudaMemcpyHostToDevice, stream));
     CK(cudaMemcpyAsync(d.pair + h.pair_base, pair.data(), pair.size() * sizeof(float2),
                        cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     return DEM_OK;
 }
 
@@ -1192,7 +1221,7 @@ int World::build(const std::vector<const dem_scene *> &scenes, const std::vector
         int32_t c3 = scenes[s]->coll_cont[3];
         CK(cudaMemcpyAsync(d.cc3 + s, &c3, 4, cudaMemcpyHostToDevice, stream));
     }
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     rc = push_det();
     if (rc) return rc;
     update_kernel_form();
@@ -1305,7 +1334,7 @@ int World::build_capacity(long long particles, long long cells, long long bonds,
         rc = push_active(s, false, 0);
         if (rc) return rc;
     }
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     rc = push_det();
     if (rc) return rc;
     return force_rebuild();
@@ -1391,7 +1420,7 @@ int World::retire(int s) {
     int rc = push_active(s, false, 0);
     if (rc) return rc;
     launch_mark_free(d, h.particle_base, h.n, free_slot, stream);
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     a_part.release(h.particle_base, h.n);
     a_cell.release(h.cell_base, h.n_cells);
     a_bond.release(h.bond_base, h.n_bonds);
@@ -1580,7 +1609,7 @@ void World::set_timing(bool on) {
 
 int World::kernel_time(int kind, double *ms, long long *n) {
     if (kind < 0 || kind >= N_TIMERS) return fail(DEM_E_INVALID, "unknown kernel");
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     Timer &t = timers[kind];
     for (size_t k = 0; k + 1 < t.ev.size(); k += 2) {
         float x = 0.0f;
@@ -1952,9 +1981,29 @@ void World::update_split() {
 // 62 / 70; a batch of 64 scenes 52 / 63), two steps are faster as a run (65 /
 // 47, 70 / 53, 84 / 74, 106 / 102).  After a run the first launch costs a
 // rebuild (~100 us), so single steps stay runs until SINGLES of them came in a row.
-constexpr int SINGLES = 32;
+//
+// While other worlds have steps queued, a run whose blocks leave no room for
+// another's on their SM has the device to itself at its barriers as well,
+// where launches of several worlds overlap.  Contexts on threads of their own,
+// microseconds a step of all by launches and by runs: 4 x 30,011 particles 28 /
+// 35, 8 x 30,011 56 / 70, 3 x 50,000 29 / 38, 4 x 77,000 34 / 56, 2 x 100,000
+// 30 / 40, 4 x 100,000 36 / 79, 2 x 262,144 50 / 69; fewer of them, or smaller
+// ones, gain from runs (2 x 30,011 26 / 18, 8 x 16,384 62 / 35).  So such a
+// world takes launches while the queued worlds hold more than 512 particles an
+// SM with it, and for HOLD calls after, since the way back costs a rebuild.
+constexpr int SINGLES = 32, HOLD = 16;
+bool World::device_full() const {
+    const long long others = queued_on(device) - queued;
+    return run_block > NARROW_BLOCK && others > 0 && others + d.N > 512LL * device_sms();
+}
+
 bool World::take_run(int n_steps) {
     if (!runs_resident()) return false;
+    if (device_full()) hold = HOLD;
+    if (hold > 0) {
+        --hold;
+        return false;
+    }
     if (n_steps != 1) {
         singles = 0;
         return true;
@@ -1996,6 +2045,7 @@ int World::step(int n_steps) {
     const bool run = take_run(n_steps);
     rc = refresh_graphs(run);
     if (rc) return rc;
+    count_queued();
     if (run) {
         if (run_steps(n_steps, RunRecord{})) return DEM_OK;
         rc = refresh_graphs(false);
@@ -2050,12 +2100,12 @@ int World::fail_waits() {
     const uint32_t next = 2u, skew = 512u;  // 512: never the number of blocks (at most one an SM)
     CK(cudaMemcpyAsync(&d.run->fail, &next, sizeof next, cudaMemcpyHostToDevice, stream));
     CK(cudaMemcpyAsync(&d.run->skew, &skew, sizeof skew, cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     return DEM_OK;
 }
 
 int World::sync() {
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     const int rc = runs_intact();
     if (rc) return rc;
     int32_t e = 0;
@@ -2211,7 +2261,7 @@ int World::download_many(const int32_t *idx, dem_scene *const *outs, int count) 
             CK(cudaGetLastError());
         }
         cudaError_t ce = fetch_bonds();
-        const cudaError_t se = cudaStreamSynchronize(stream);  // the copies write the callers' arrays until then
+        const cudaError_t se = wait();  // the copies write the callers' arrays until then
         if (ce == cudaSuccess) ce = se;
         if (ce != cudaSuccess) return fail(DEM_E_CUDA, cudaGetErrorString(ce));
         rc = first_error();
@@ -2284,6 +2334,7 @@ int World::download_many(const int32_t *idx, dem_scene *const *outs, int count) 
         pipe.release(c);
     }
     pipe.join();
+    settled();
     return DEM_OK;
 }
 
@@ -2312,7 +2363,7 @@ int World::set_properties(int s, int32_t *selections, const int32_t *props) {
     cudaMemcpyAsync(dprops, props, sizeof(int32_t) * 28, cudaMemcpyHostToDevice, stream);
     launch_set_properties(d, s, dsel, dout, dprops, block, stream);
     cudaError_t e = cudaMemcpyAsync(selections, dout, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, stream);
-    cudaError_t e2 = cudaStreamSynchronize(stream);
+    cudaError_t e2 = wait();
     cudaFree(dsel);
     cudaFree(dout);
     cudaFree(dprops);
@@ -2361,7 +2412,7 @@ int World::fixity_event(int s, int kind, int32_t *selections, int throw_vel, flo
     CK(cudaMalloc(&dbuf, sizeof(int32_t) * (size_t)k));
     cudaMemcpyAsync(dbuf, idx.data(), sizeof(int32_t) * k, cudaMemcpyHostToDevice, stream);
     launch_fixity_event(d, h.particle_base, dbuf, k, kind, vx, vy, set_vel, stream);
-    const cudaError_t e = cudaStreamSynchronize(stream);
+    const cudaError_t e = wait();
     cudaFree(dbuf);
     if (e != cudaSuccess) return fail(DEM_E_CUDA, std::string("fixity event: ") + cudaGetErrorString(e));
     return runs_intact();
@@ -2388,7 +2439,7 @@ int World::get_datum(int s, const int32_t *selections, double out[10]) {
     cudaMemcpyAsync(d_idx, idx.data(), sizeof(int32_t) * k, cudaMemcpyHostToDevice, stream);
     launch_gather_datum(d, h.particle_base, d_idx, k, d_out, stream);
     cudaMemcpyAsync(f.data(), d_out, sizeof(float) * 10 * (size_t)k, cudaMemcpyDeviceToHost, stream);
-    const cudaError_t e = cudaStreamSynchronize(stream);
+    const cudaError_t e = wait();
     cudaFree(dbuf);
     if (e != cudaSuccess) return fail(DEM_E_CUDA, std::string("datum: ") + cudaGetErrorString(e));
     const int rc = runs_intact();
@@ -2459,7 +2510,7 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
         if (d_sel) {
             rc = runs_intact();
             if (rc == DEM_OK && !run_steps(m, RunRecord{d_sel, s, h.particle_base, (int)per, d_rows})) {
-                cudaStreamSynchronize(stream);  // the rest by launches
+                wait();  // the rest by launches
                 cudaFree(dbuf);
                 return record(s, selections, n_steps - s0, rows + 10LL * s0);
             }
@@ -2470,7 +2521,7 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
         }
         if (rc) break;
         e = cudaMemcpyAsync(f.data(), d_rows, sizeof(float) * (size_t)(per * m), cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        if (e == cudaSuccess) e = wait();
         if (e != cudaSuccess) {
             rc = fail(DEM_E_CUDA, std::string("record: ") + cudaGetErrorString(e));
             break;
@@ -2486,13 +2537,13 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
             for (int q = 0; q < 10; ++q) out[q] = q == 6 ? sums[q] : sums[q] / (double)k;
         }
     }
-    cudaStreamSynchronize(stream);
+    wait();
     cudaFree(dbuf);
     return rc ? rc : k;
 }
 
 int World::drain_events(std::vector<dem_break_event> &out) {
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     const int rc = runs_intact();
     if (rc) return rc;
     unsigned long long cnt = 0;
@@ -2525,14 +2576,14 @@ int World::broad_phase_snapshot(int s, int32_t *keys, int32_t *order, int32_t *c
     std::vector<uint32_t> k(n);
     std::vector<int32_t> srt(n), orig(n), cs((size_t)h.n_cells + 1);
     CK(cudaMemcpyAsync(cs.data(), d.cell_start + h.cell_base, cs.size() * 4, cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     const int first = cs[0];
     if (n > 0) {
         CK(cudaMemcpyAsync(k.data(), d.keys + base, n * 4, cudaMemcpyDeviceToHost, stream));
         CK(cudaMemcpyAsync(srt.data(), d.sorted + first, n * 4, cudaMemcpyDeviceToHost, stream));
         CK(cudaMemcpyAsync(orig.data(), d.orig + base, n * 4, cudaMemcpyDeviceToHost, stream));
     }
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     for (int i = 0; i < n; ++i) {
         if (keys) keys[orig[i]] = std::min((int32_t)k[i] - h.cell_base, grid_cells);
         int src = srt[i] - base;
@@ -2548,7 +2599,7 @@ int World::broad_phase_snapshot(int s, int32_t *keys, int32_t *order, int32_t *c
 }
 
 int World::stats(dem_stats *out) {
-    CK(cudaStreamSynchronize(stream));
+    CK(wait());
     unsigned long long st[6];
     CK(cudaMemcpy(st, d.stats, sizeof st, cudaMemcpyDeviceToHost));
     int32_t e = 0;

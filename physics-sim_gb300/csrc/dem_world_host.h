@@ -136,6 +136,7 @@ class World {
     int kernel_time(int kind, double *ms, long long *n);
     void set_timing(bool on);
     int fail_waits();  // debug
+    static long long queued_on(int device);  // particles of the worlds with steps queued (DEVICES at most)
     long long run_calls = 0;       // step calls (and chunks of a record) taken as runs
     int set_runs(int mode);        // debug: 0 the library's choice, 1 launches, 2 every run refused
 
@@ -171,6 +172,14 @@ class World {
     bool run_steps(int n_steps, const RunRecord &rec);
     int refresh_graphs(bool run);
     bool take_run(int n_steps);
+    bool device_full() const;
+    int hold = 0;                  // step calls that stay launches
+    // the world's particles while it has steps queued that no call has waited
+    // for, counted on its device
+    long long queued = 0;
+    void count_queued();
+    cudaError_t wait();            // for the stream
+    void settled();
     int singles = 0;               // step calls of one step in a row, while they are runs
     RunReport *report = nullptr;   // page-locked (StepRun::report)
     int runs_intact();

@@ -1,6 +1,7 @@
 """Which step calls are runs: calls of several steps, but not calls of one step
 (a launch a step is faster there) unless a run has just left the cell table
-behind.  The results do not depend on it."""
+behind, and not in large worlds while other worlds have steps queued.  The
+results do not depend on it."""
 import numpy as np
 import pytest
 
@@ -55,3 +56,73 @@ def test_records_are_one_run_or_launches(n, runs):
         assert ctx.run_calls() - before == runs + 1
         oracle.step(ref, p, 7)
         assert_same_state(ctx.download(), ref)
+
+
+def test_wide_runs_leave_the_device_to_others():
+    n = 90000
+    sc, p, ext = shaken_bed(n, 7)
+    ref = copy_scene(sc)
+    small = shaken_bed(5000, 1)
+    with dem.Context(copy_scene(sc), p, **ext) as a, dem.Context(copy_scene(sc), p, **ext) as b, \
+            dem.Context(small[0], small[1]) as c:
+        done = [0, 0]
+
+        def both(k, steps, runs):
+            ctx = (a, b)[k]
+            before = ctx.run_calls()
+            ctx.step(steps)
+            done[k] += steps
+            assert ctx.run_calls() - before == runs
+
+        both(0, 20, 1)          # alone
+        both(1, 20, 0)          # a's steps are queued
+        c.step(20)              # a grid that shares the SMs is a run all the same
+        assert c.run_calls() == 1
+        a.synchronize()
+        c.download()
+        for _ in range(15):     # b stays on launches for a while
+            both(1, 3, 0)
+        both(1, 3, 1)
+        both(0, 3, 0)           # now b's are queued
+        b.break_events()
+        for _ in range(15):
+            both(0, 3, 0)
+        both(0, 3, 1)
+        a.synchronize()
+        d = dem.Context(copy_scene(sc), p, **ext)
+        d.step(2)
+        d.close()               # a world that is gone counts no more
+        both(1, 5, 1)
+        oracle.step(ref, p, min(done))
+        for k in (0, 1):
+            rest = max(done) - done[k]
+            if rest:
+                (a, b)[k].step(rest)
+        oracle.step(ref, p, max(done) - min(done))
+        for ctx in (a, b):
+            assert_same_state(ctx.download(), ref)
+
+
+def test_large_worlds_on_threads_of_their_own():
+    import threading
+
+    sc, p, ext = shaken_bed(100000, 9)
+    ref = copy_scene(sc)
+    oracle.step(ref, p, 60)
+    got = []
+
+    def work():
+        with dem.Context(copy_scene(sc), p, **ext) as ctx:
+            for steps in (20, 1, 19, 20):
+                ctx.step(steps)
+                ctx.synchronize()
+            got.append(ctx.download())
+
+    threads = [threading.Thread(target=work) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(got) == 4
+    for g in got:
+        assert_same_state(g, ref)
