@@ -1198,6 +1198,7 @@ __global__ void k_rebuild_done(DevWorld w, const int32_t *gate) {
     w.run->linked = 0;
     const unsigned long long n = w.stats[4] + 1ull;
     w.stats[4] = n;
+    report_lists(w);
     // the next rebuild reorders when it is the first of a new group of reorder_every
     *w.reorder = (w.reorder_every <= 1 || n % (unsigned long long)w.reorder_every == 0ull) ? 1 : 0;
 }

@@ -19,6 +19,7 @@ __global__ void k_run_begin(DevWorld w, int todo, const int32_t *rec_rows, int r
     R.rec_base = rec_base;
     R.rec_per = rec_per;
     R.rec_out = rec_out;
+    report_lists(w);
 }
 
 void launch_run_begin(const DevWorld &w, int todo, const RunRecord &rec, cudaStream_t st) {

@@ -135,11 +135,13 @@ struct StepRun {
     float *rec_out;
     uint32_t skew;           // the barrier counters' start, 0; else no barrier is ever complete (tests)
     struct RunReport *report;
+    unsigned long long rebuilds, overflows;  // DevWorld::stats [4] and [5] when the report was last written
 };
 // What the host learns of the runs without a copy: words in page-locked host
 // memory that the device writes, read after the stream has been waited for.
 struct RunReport {
-    int32_t failed;  // a wait gave up: the world's state is of no step
+    int32_t failed;       // a wait gave up: the world's state is of no step
+    uint32_t overflows;   // particles whose list overflowed, a rebuild, of the latest rebuilds known
 };
 // before every launch of the kernel
 __device__ __forceinline__ void clear_run_barrier(StepRun &R) {
@@ -215,6 +217,16 @@ struct DevWorld {
     int32_t *act;               // [S] 1 = the scene steps; 0 = frozen (finished or free slot)
     long long *remaining;       // [S] steps left before the scene freezes (served scenes)
 };
+
+// by one thread, with no list build under way
+__device__ __forceinline__ void report_lists(const DevWorld &w) {
+    StepRun &R = *w.run;
+    const unsigned long long rebuilds = w.stats[4], overflows = w.stats[5];
+    if (rebuilds == R.rebuilds) return;
+    *(volatile uint32_t *)&R.report->overflows = (uint32_t)((overflows - R.overflows) / (rebuilds - R.rebuilds));
+    R.rebuilds = rebuilds;
+    R.overflows = overflows;
+}
 
 // ---- stateless detection schedule -----------------------------------------
 // The LOM pass's thread 0 does cc1 += 1; if cc1 >= interval {cc0 = 1; cc1 = 0}

@@ -1997,9 +1997,24 @@ bool World::device_full() const {
     return run_block > NARROW_BLOCK && others > 0 && others + d.N > 512LL * device_sms();
 }
 
+// Where most lists overflow their particles go over whole cells at every step:
+// launches read the partners through L1, a run only through L2, and its
+// rebuilds walk chains (microseconds a step by launches and by runs, disks
+// overlapping 5 to 10 deep: 3,000 462 / 534, 30,000 1,042 / 1,173, 100,000 692 /
+// 963, 250,000 2,101 / 3,975; packs of sizes 1 to 5 with 0.5 % of the lists
+// full 187 / 66 at 30,000 and 233 / 207 at 250,000).
+bool World::crowded() const {
+    const long long over = report ? *(volatile uint32_t *)&report->overflows : 0;
+    if (over == 0) return false;
+    long long n = 0;
+    for (const auto &h : sh)
+        if (h.active) n += h.n;
+    return 2 * over > n;
+}
+
 bool World::take_run(int n_steps) {
     if (!runs_resident()) return false;
-    if (device_full()) hold = HOLD;
+    if (device_full() || crowded()) hold = HOLD;
     if (hold > 0) {
         --hold;
         return false;
@@ -2016,13 +2031,11 @@ bool World::take_run(int n_steps) {
 int World::refresh_graphs(bool run) {
     update_param_source();
     update_split();
-    // the records of a world that runs resident sit in L2 wherever they are:
-    // its rebuilds stay within the run, all but one in 32
-    const int every = reorder_every > 0 ? reorder_every : runs_resident() ? 32 : (sh.size() == 1 ? 3 : 8);
-    if (every != d.reorder_every) {
-        d.reorder_every = every;
-        drop_graph();
-    }
+    // the records of a run sit in L2 wherever they are: its rebuilds stay within
+    // it, all but one in 32.  Each graph is captured with the interval of its
+    // own route (crowded worlds by launches with 32 and with 3, microseconds a
+    // step: 100,000 particles 826 / 694, 250,000 2,548 / 2,108)
+    d.reorder_every = reorder_every > 0 ? reorder_every : run ? 32 : (sh.size() == 1 ? 3 : 8);
     if (was_resident && !run) {
         // the cell table may be of an earlier rebuild than the lists
         const int rc = force_rebuild(false);

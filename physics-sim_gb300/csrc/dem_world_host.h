@@ -173,6 +173,7 @@ class World {
     int refresh_graphs(bool run);
     bool take_run(int n_steps);
     bool device_full() const;
+    bool crowded() const;
     int hold = 0;                  // step calls that stay launches
     // the world's particles while it has steps queued that no call has waited
     // for, counted on its device

@@ -1,11 +1,12 @@
 """Which step calls are runs: calls of several steps, but not calls of one step
 (a launch a step is faster there) unless a run has just left the cell table
-behind, and not in large worlds while other worlds have steps queued.  The
-results do not depend on it."""
+behind, not in large worlds while other worlds have steps queued, and not
+while most candidate lists are full.  The results do not depend on it."""
 import numpy as np
 import pytest
 
 import dem
+import dem_scenes
 import oracle
 from gpu_backend import assert_same_state, copy_scene
 from test_gpu_steps import shaken_bed
@@ -15,7 +16,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n", [128, 700, 5000, 90000])
 def test_calls_of_one_step_are_launches(n):
-    sc, p, _ = shaken_bed(n, 5, speed=4.0, spacing=1.1)  # full lists, which search the cell table
+    sc, p, _ = shaken_bed(n, 5, speed=4.0, spacing=1.1)  # some lists full, which search the cell table
     ref = copy_scene(sc)
     with dem.Context(copy_scene(sc), p) as ctx:
         def calls(count, steps):
@@ -126,3 +127,30 @@ def test_large_worlds_on_threads_of_their_own():
     assert len(got) == 4
     for g in got:
         assert_same_state(g, ref)
+
+
+@pytest.mark.parametrize("n", [900, 6000, 90000])
+def test_crowded_worlds_take_launches(n):
+    """Disks that overlap several deep and fly apart: launches while most lists
+    are full, runs again once they are not."""
+    sc, p, _ = shaken_bed(n, 5, speed=1.0, spacing=0.5)
+    p = dict(p, gravity=0, hor_bound=8 * p["hor_bound"], vert_bound=8 * p["vert_bound"])
+    sc["grid"] = dem_scenes.grid_capacity(p["hor_bound"], p["vert_bound"], sc["radii"], n)
+    sc["vel"][:] = 20.0 * sc["pos"]
+    ref = copy_scene(sc)
+    with dem.Context(copy_scene(sc), p) as ctx:
+        calls = []
+        for k in range(60):
+            before = ctx.run_calls()
+            ctx.step(3 if k < 6 else 30)
+            if k < 6:
+                oracle.step(ref, p, 3)
+                ctx.synchronize()
+            if k == 5:
+                assert_same_state(ctx.download(), ref)
+                assert ctx.stats()["list_overflows"] > n // 2
+            calls.append(ctx.run_calls() - before)
+        ctx.synchronize()
+    assert calls[0] == 1, "nothing is known before the first rebuild"
+    assert calls[2:6] == [0, 0, 0, 0], "most lists are full"
+    assert calls[-1] == 1, "the disks have flown apart"
