@@ -316,7 +316,11 @@ void *dem_batch_stream(dem_batch *b);
  * 0.45 r_max: how often particles are re-sorted by cell), the particle-kernel
  * block size (128, 256, 512), the steps per captured graph (21, 35, 70),
  * whether the Simulation pass runs as one kernel or two (split_narrow) and
- * whether it carries the next step's LOM pass (unfused_lom).
+ * whether it carries the next step's LOM pass (unfused_lom).  The trials step
+ * the way the whole batch will; the last four knobs, which change nothing in a
+ * batch that takes a step call in one kernel (see dem_ext.reorder_interval),
+ * and split_narrow where the library chooses two kernels by itself, are then
+ * left at their defaults without a trial.
  * Copy the result's six fields into each scene's dem_ext. */
 typedef struct dem_tune_result {
     float search_cell_factor;

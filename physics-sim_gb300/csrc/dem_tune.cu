@@ -8,11 +8,15 @@
 // depend on the scenes and the GPU.
 // dem_batch_autotune times short runs of a sample of the batch's scenes with
 // candidate values, one knob at a time (coordinate descent from the library
-// defaults), and returns the fastest combination as dem_ext fields.
+// defaults), and returns the fastest combination as dem_ext fields.  Trials
+// step the way the batch will: by launches when the batch is too large for
+// runs, however small the sample; and in runs, or where the library's choice
+// is two kernels already, the knobs that change nothing are left alone.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -39,9 +43,14 @@ struct Knobs {
 };
 
 // ms per step of the sample with the given knobs: warm run (graph capture,
-// first rebuild), then `steps` timed steps with events on the world's stream
+// first rebuild), then `steps` timed steps with events on the world's stream.
+// launches: by launches whatever the sample's size; how: the way it stepped.
+struct How {
+    bool runs = false, split = false;
+};
 int trial(const std::vector<const dem_scene *> &sc, const std::vector<dem_params> &ps,
-          const std::vector<dem_ext> &base, const Knobs &k, int steps, double *ms_per_step) {
+          const std::vector<dem_ext> &base, const Knobs &k, int steps, bool launches, double *ms_per_step,
+          How *how = nullptr) {
     std::vector<dem_ext> es = base;
     for (auto &e : es) {
         e.search_cell_factor = k.cell_factor;
@@ -63,7 +72,9 @@ int trial(const std::vector<const dem_scene *> &sc, const std::vector<dem_params
         cudaGetDevice(&w.device);
         rc = w.build(sc, ps, es);
         cudaEvent_t e0 = nullptr, e1 = nullptr;
+        if (rc == DEM_OK && launches) rc = w.set_runs(1);
         if (rc == DEM_OK) rc = w.step(steps);
+        if (how) *how = How{w.runs_resident(), w.d.split != 0};
         if (rc == DEM_OK && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
             rc = tfail(DEM_E_CUDA, "event creation failed");
         if (rc == DEM_OK) {
@@ -137,13 +148,15 @@ int dem_batch_autotune(const dem_scene *const *scenes, const dem_params *params,
     Knobs best;
     double best_ms = 0.0;
     int trials = 0;
-    int rc = trial(sc, ps, es, best, trial_steps, &best_ms);
+    const bool launches = total > INT_MAX || demgb::steps_block((int)total) == 0;
+    How how;
+    int rc = trial(sc, ps, es, best, trial_steps, launches, &best_ms, &how);
     if (rc) return rc;
     ++trials;
     const double default_ms = best_ms;
     auto try_knobs = [&](const Knobs &k) -> int {
         double ms = 0.0;
-        int r = trial(sc, ps, es, k, trial_steps, &ms);
+        int r = trial(sc, ps, es, k, trial_steps, launches, &ms);
         if (r) return r;
         ++trials;
         if (ms < best_ms) {
@@ -152,36 +165,37 @@ int dem_batch_autotune(const dem_scene *const *scenes, const dem_params *params,
         }
         return DEM_OK;
     };
+    const Knobs first;  // a knob's default has been timed with the best of the knobs before it
     for (float v : skins) {
-        if (v == best.skin) continue;
+        if (v == first.skin) continue;
         Knobs k = best;
         k.skin = v;
         if ((rc = try_knobs(k))) return rc;
     }
     for (float v : cells) {
-        if (v == best.cell_factor) continue;
+        if (v == first.cell_factor) continue;
         Knobs k = best;
         k.cell_factor = v;
         if ((rc = try_knobs(k))) return rc;
     }
     for (int v : blocks) {
-        if (v == best.block) continue;
+        if (v == first.block || how.runs) continue;
         Knobs k = best;
         k.block = v;
         if ((rc = try_knobs(k))) return rc;
     }
     for (int v : graphs) {
-        if (v == best.graph_steps) continue;
+        if (v == first.graph_steps || how.runs) continue;
         Knobs k = best;
         k.graph_steps = v;
         if ((rc = try_knobs(k))) return rc;
     }
-    {
+    if (!how.runs && !how.split) {
         Knobs k = best;
         k.split = 1 - best.split;
         if ((rc = try_knobs(k))) return rc;
     }
-    {
+    if (!how.runs) {
         Knobs k = best;
         k.unfused = 1 - best.unfused;
         if ((rc = try_knobs(k))) return rc;

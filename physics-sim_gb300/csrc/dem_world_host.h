@@ -137,6 +137,7 @@ class World {
     void set_timing(bool on);
     int fail_waits();  // debug
     static long long queued_on(int device);  // particles of the worlds with steps queued (DEVICES at most)
+    bool runs_resident() const;    // step calls may be runs
     long long run_calls = 0;       // step calls (and chunks of a record) taken as runs
     int set_runs(int mode);        // debug: 0 the library's choice, 1 launches, 2 every run refused
 
@@ -165,7 +166,6 @@ class World {
     int run_block = 0;             // block size of a resident run (steps_block), 0: none
     cudaGraphExec_t graph_run[2] = {nullptr, nullptr};  // a run of steps, per buffer parity
     int capture_run(cudaGraphExec_t *out);
-    bool runs_resident() const;
     bool runs_refused = false;     // a run could not be captured or launched: launches from then on
     bool runs_off = false, runs_fault = false;  // debug (set_runs)
     bool ready_run();
