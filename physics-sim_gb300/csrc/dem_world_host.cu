@@ -74,7 +74,8 @@ void RangeAlloc::release(long long off, long long n) {
 
 // Particles of the worlds whose step calls no call has waited for, by device:
 // what the runs of other worlds would share the device with.  A host that
-// only ever waits for a world's stream by itself leaves the world counted.
+// only ever waits for a world's stream by itself leaves the world counted;
+// worlds of plain launches, which such hosts capture, are not.
 constexpr int DEVICES = 64;
 static std::atomic<long long> queued_particles[DEVICES];
 
@@ -83,7 +84,7 @@ long long World::queued_on(int device) {
 }
 
 void World::count_queued() {
-    if (queued || device < 0 || device >= DEVICES) return;
+    if (queued || !use_graphs || device < 0 || device >= DEVICES) return;
     queued = d.N;
     queued_particles[device].fetch_add(queued, std::memory_order_relaxed);
 }

@@ -94,6 +94,9 @@ def test_wide_runs_leave_the_device_to_others():
         d.step(2)
         d.close()               # a world that is gone counts no more
         both(1, 5, 1)
+        with dem.Context(copy_scene(sc), p, plain_launches=1, **ext) as d:
+            d.step(2)           # nor one whose launches the host may capture
+            both(1, 5, 1)
         oracle.step(ref, p, min(done))
         for k in (0, 1):
             rest = max(done) - done[k]
