@@ -2408,6 +2408,7 @@ __global__ void __launch_bounds__(ST_THREADS) k_stage_out(DevWorld w, RefArrays 
     __shared__ uint32_t s_mask[ST_P];
     const long long t0 = (long long)blockIdx.x * ST_P;
     const int np = (int)min((long long)ST_P, total - t0);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && w.run->fail == 1u) atomicOr(err + count, 64);
     tile_items(it, count, t0, np, s_item, s_g);
     if (threadIdx.x < np) {
         const int k = s_item[threadIdx.x], g = s_g[threadIdx.x];
@@ -2498,8 +2499,8 @@ void launch_stage_out(const DevWorld &w, const RefArrays &r, const StageItem *it
 // words, both coalesced
 constexpr int COPY_THREADS = 256;
 __global__ void __launch_bounds__(COPY_THREADS) k_copies(const HostCopy *__restrict__ c, int n,
-                                                          const int32_t *guard, const uint32_t *guard2) {
-    if (guard && (*guard != 0 || *guard2 == 1u)) return;
+                                                          const int32_t *guard) {
+    if (guard && *guard) return;
     __shared__ int s_k;
     const long long b = blockIdx.x;
     if (threadIdx.x == 0) {
@@ -2535,10 +2536,9 @@ __global__ void __launch_bounds__(COPY_THREADS) k_copies(const HostCopy *__restr
     }
 }
 
-void launch_copies(const HostCopy *c, int n, long long pieces, const int32_t *guard, const uint32_t *guard2,
-                   cudaStream_t st) {
+void launch_copies(const HostCopy *c, int n, long long pieces, const int32_t *guard, cudaStream_t st) {
     if (n <= 0 || pieces <= 0) return;
-    k_copies<<<(unsigned)pieces, COPY_THREADS, 0, st>>>(c, n, guard, guard2);
+    k_copies<<<(unsigned)pieces, COPY_THREADS, 0, st>>>(c, n, guard);
 }
 
 // ------------------------------------------------------- Fix / Drop / Release

@@ -19,6 +19,7 @@ __global__ void k_run_begin(DevWorld w, int todo, const int32_t *rec_rows, int r
     R.rec_base = rec_base;
     R.rec_per = rec_per;
     R.rec_out = rec_out;
+    if (R.fail == 1u) *(volatile int32_t *)&R.report->failed = 1;
     report_lists(w);
 }
 

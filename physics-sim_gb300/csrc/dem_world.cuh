@@ -137,11 +137,11 @@ struct StepRun {
     struct RunReport *report;
     unsigned long long rebuilds, overflows;  // DevWorld::stats [4] and [5] when the report was last written
 };
-// What the host learns of the runs without a copy: words in page-locked host
-// memory that the device writes, read after the stream has been waited for.
+// What the host learns of the runs, in page-locked host memory.
 struct RunReport {
-    int32_t failed;       // a wait gave up: the world's state is of no step
-    uint32_t overflows;   // particles whose list overflowed, a rebuild, of the latest rebuilds known
+    int32_t err;          // DevWorld::err as of the last wait for the stream (World::queue_check)
+    int32_t failed;       // written by the device: a run before this one failed
+    uint32_t overflows;   // by the device: particles whose list overflowed, a rebuild, of the latest rebuilds known
 };
 // before every launch of the kernel
 __device__ __forceinline__ void clear_run_barrier(StepRun &R) {
@@ -372,7 +372,8 @@ void launch_stage_check(const RefArrays &r, const StageItem *items, int count, l
 void launch_stage_in(const DevWorld &w, const RefArrays &r, const StageItem *items, int count, long long total,
                      cudaStream_t st);
 // internal layout -> reference layout; err[k] bits: 16 internal map corrupt,
-// 32 contact partner outside the scene; err[count] = OR of all
+// 32 contact partner outside the scene; err[count] = OR of all, and 64 after a
+// failed run (StepRun::fail)
 void launch_stage_out(const DevWorld &w, const RefArrays &r, const StageItem *items, int count, long long total,
                       int32_t *err, cudaStream_t st);
 
@@ -388,9 +389,8 @@ struct HostCopy {
     long long piece0;
 };
 // every piece of copies c[0..n) (`pieces` in all); nothing if guard != NULL
-// and *guard != 0 or *guard2 == 1 (StepRun::fail)
-void launch_copies(const HostCopy *c, int n, long long pieces, const int32_t *guard, const uint32_t *guard2,
-                   cudaStream_t st);
+// and *guard != 0
+void launch_copies(const HostCopy *c, int n, long long pieces, const int32_t *guard, cudaStream_t st);
 
 // Fix / Drop / Release events (src/shaders/event_handling/{Fix,Drop,Release}.wgsl)
 // on `count` particles of the scene whose first particle is `base`, given

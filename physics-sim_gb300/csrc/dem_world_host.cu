@@ -101,6 +101,15 @@ cudaError_t World::wait() {
     return e;
 }
 
+// the device's error word for runs_intact() after the next wait; ahead of a
+// call's own copies, which then hide most of it (3 us; behind them 7).  Only
+// runs wait between blocks.
+cudaError_t World::queue_check() {
+    if (!unchecked) return cudaSuccess;
+    unchecked = false;
+    return cudaMemcpyAsync(&report->err, d.err, sizeof report->err, cudaMemcpyDeviceToHost, stream);
+}
+
 World::~World() {
     settled();
     set_timing(true);
@@ -1012,7 +1021,7 @@ int World::stage_many(const int32_t *idx, const dem_scene *const *scs, int count
         if (nc > 0) {
             ce = cudaMemcpyAsync(d_copies, hc, sizeof(HostCopy) * nc, cudaMemcpyHostToDevice, stream);
             if (ce == cudaSuccess) {
-                launch_copies(d_copies, nc, pieces, nullptr, nullptr, stream);
+                launch_copies(d_copies, nc, pieces, nullptr, stream);
                 ce = cudaGetLastError();
             }
         }
@@ -1902,6 +1911,7 @@ bool World::run_steps(int n_steps, const RunRecord &rec) {
         return false;
     }
     ++run_calls;
+    unchecked = true;
     launches += 2;
     host_step += n_steps;
     return true;
@@ -2102,10 +2112,11 @@ int World::step(int n_steps) {
 }
 
 // After a wait that gave up the state is of no step and nothing steps any
-// more: the calls that wait for the stream and those that step say so.  The
-// device has set the word by the time a wait for the stream returns.
+// more: the calls that wait for the stream say so at once (queue_check, a
+// download by its check words), and those that step once one of them or a
+// later run has told.
 int World::runs_intact() {
-    if (!report || *(volatile int32_t *)&report->failed == 0) return DEM_OK;
+    if (!report || !((report->err & 8) || *(volatile int32_t *)&report->failed)) return DEM_OK;
     return fail(DEM_E_TIMEOUT, "a wait between the blocks of a step kernel gave up; create the world anew");
 }
 
@@ -2119,11 +2130,12 @@ int World::fail_waits() {
 }
 
 int World::sync() {
+    unchecked = true;  // the other errors come from launches too
+    CK(queue_check());
     CK(wait());
     const int rc = runs_intact();
     if (rc) return rc;
-    int32_t e = 0;
-    CK(cudaMemcpy(&e, d.err, 4, cudaMemcpyDeviceToHost));
+    const int32_t e = report->err;
     if (e) return fail(DEM_E_STATE, "device error flags set: " + std::to_string(e));
     return DEM_OK;
 }
@@ -2241,6 +2253,7 @@ int World::download_many(const int32_t *idx, dem_scene *const *outs, int count) 
         out->grid = h.grid;
     };
     auto first_error = [&]() -> int {
+        if (nt > 0 && (h_err[nt] & 64)) report->err |= 8;
         const int r1 = runs_intact();
         if (r1) return r1;
         for (int i = 0; i < nt; ++i)
@@ -2271,7 +2284,7 @@ int World::download_many(const int32_t *idx, dem_scene *const *outs, int count) 
         }
         if (nc > 0) {
             CK(cudaMemcpyAsync(d_copies, hc, sizeof(HostCopy) * nc, cudaMemcpyHostToDevice, stream));
-            launch_copies(d_copies, nc, pieces, d_item_err + nt, &d.run->fail, stream);
+            launch_copies(d_copies, nc, pieces, d_item_err + nt, stream);
             CK(cudaGetLastError());
         }
         cudaError_t ce = fetch_bonds();
@@ -2376,6 +2389,7 @@ int World::set_properties(int s, int32_t *selections, const int32_t *props) {
     cudaMemcpyAsync(dout, selections, sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream);
     cudaMemcpyAsync(dprops, props, sizeof(int32_t) * 28, cudaMemcpyHostToDevice, stream);
     launch_set_properties(d, s, dsel, dout, dprops, block, stream);
+    queue_check();
     cudaError_t e = cudaMemcpyAsync(selections, dout, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, stream);
     cudaError_t e2 = wait();
     cudaFree(dsel);
@@ -2426,6 +2440,7 @@ int World::fixity_event(int s, int kind, int32_t *selections, int throw_vel, flo
     CK(cudaMalloc(&dbuf, sizeof(int32_t) * (size_t)k));
     cudaMemcpyAsync(dbuf, idx.data(), sizeof(int32_t) * k, cudaMemcpyHostToDevice, stream);
     launch_fixity_event(d, h.particle_base, dbuf, k, kind, vx, vy, set_vel, stream);
+    queue_check();
     const cudaError_t e = wait();
     cudaFree(dbuf);
     if (e != cudaSuccess) return fail(DEM_E_CUDA, std::string("fixity event: ") + cudaGetErrorString(e));
@@ -2452,6 +2467,7 @@ int World::get_datum(int s, const int32_t *selections, double out[10]) {
     float *d_out = reinterpret_cast<float *>(d_idx + k);
     cudaMemcpyAsync(d_idx, idx.data(), sizeof(int32_t) * k, cudaMemcpyHostToDevice, stream);
     launch_gather_datum(d, h.particle_base, d_idx, k, d_out, stream);
+    queue_check();
     cudaMemcpyAsync(f.data(), d_out, sizeof(float) * 10 * (size_t)k, cudaMemcpyDeviceToHost, stream);
     const cudaError_t e = wait();
     cudaFree(dbuf);
@@ -2534,6 +2550,7 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
             if (rc == DEM_OK) launch_gather_datum(d, h.particle_base, d_idx, k, d_rows + per * j, stream);
         }
         if (rc) break;
+        queue_check();
         e = cudaMemcpyAsync(f.data(), d_rows, sizeof(float) * (size_t)(per * m), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = wait();
         if (e != cudaSuccess) {
@@ -2557,11 +2574,12 @@ int World::record(int s, const int32_t *selections, int n_steps, double *rows) {
 }
 
 int World::drain_events(std::vector<dem_break_event> &out) {
+    CK(queue_check());
+    unsigned long long cnt = 0;
+    CK(cudaMemcpyAsync(&cnt, d.ev_count, sizeof cnt, cudaMemcpyDeviceToHost, stream));
     CK(wait());
     const int rc = runs_intact();
     if (rc) return rc;
-    unsigned long long cnt = 0;
-    CK(cudaMemcpy(&cnt, d.ev_count, sizeof cnt, cudaMemcpyDeviceToHost));
     size_t k = (size_t)std::min<unsigned long long>(cnt, d.ev_cap);
     out.resize(k);
     if (k) CK(cudaMemcpy(out.data(), d.ev, k * sizeof(Event), cudaMemcpyDeviceToHost));

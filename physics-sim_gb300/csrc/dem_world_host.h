@@ -181,6 +181,8 @@ class World {
     void count_queued();
     cudaError_t wait();            // for the stream
     void settled();
+    cudaError_t queue_check();
+    bool unchecked = false;        // a run since the last queue_check
     int singles = 0;               // step calls of one step in a row, while they are runs
     RunReport *report = nullptr;   // page-locked (StepRun::report)
     int runs_intact();
