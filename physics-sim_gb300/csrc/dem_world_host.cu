@@ -1851,7 +1851,8 @@ int World::capture_run(cudaGraphExec_t *out) {
         e = cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
         cudaGraph_t done = nullptr;
-        e = runs_fault ? cudaErrorCooperativeLaunchTooLarge : launch_steps(d, run_block, side, more, due, kernel_form, &par_pv, par_ps);
+        e = runs_fault ? cudaErrorCooperativeLaunchTooLarge
+                       : launch_steps(d, run_block, side, more, due, kernel_form, &par_pv, par_ps);
         const cudaGraphNode_t *deps = nullptr;
         size_t ndeps = 0;
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1910,6 +1911,7 @@ bool World::run_steps(int n_steps, const RunRecord &rec) {
         runs_refused = true;
         return false;
     }
+    count_queued();
     ++run_calls;
     unchecked = true;
     launches += 2;
@@ -2069,12 +2071,12 @@ int World::step(int n_steps) {
     const bool run = take_run(n_steps);
     rc = refresh_graphs(run);
     if (rc) return rc;
-    count_queued();
     if (run) {
         if (run_steps(n_steps, RunRecord{})) return DEM_OK;
         rc = refresh_graphs(false);
         if (rc) return rc;
     }
+    count_queued();
     int k = 0;
     if (use_graphs && !timing && n_steps > 0) {
         while (n_steps - k >= graph_steps) {
