@@ -952,6 +952,7 @@ __device__ __forceinline__ void list_build_one(const DevWorld &w, int i) {
     for (int cy = cy0; cy <= cy1; ++cy) {
         const int row = P.cell_base + cy * P.g_w;
         const int beg = w.cell_start[row + cx0], end = w.cell_start[row + cx1 + 1];
+        if (end - beg > CROWDED_ROW) w.run->crowd = 1u;
         for (int k = beg; k < end; ++k) {
             const int b = w.sorted[k];
             if (b == i) continue;
@@ -1163,9 +1164,11 @@ __global__ void __launch_bounds__(LT_THREADS) k_list_tiles(DevWorld w, const int
                 const int *cs = s_cs + hit * LT_CELLS;
                 const int at = s_off[hit] - cs[0];
                 const int beg = cs[a - s_lo[hit]] + at, fin = cs[z - s_lo[hit]] + at;
+                if (fin - beg > CROWDED_ROW) w.run->crowd = 1u;
                 for (int k = beg; k < fin; ++k) list_consider(P, i, pa, s_idx[k], s_pr[k], h, ls);
             } else {
                 const int beg = w.cell_start[a], fin = w.cell_start[z];
+                if (fin - beg > CROWDED_ROW) w.run->crowd = 1u;
                 for (int k = beg; k < fin; ++k) {
                     const int b = w.sorted[k];
                     list_consider(P, i, pa, b, w.pr[b], h, ls);
@@ -1199,6 +1202,8 @@ __global__ void k_rebuild_done(DevWorld w, const int32_t *gate) {
     const unsigned long long n = w.stats[4] + 1ull;
     w.stats[4] = n;
     report_lists(w);
+    *(volatile uint32_t *)&w.run->report->crowd = w.run->crowd;
+    w.run->crowd = 0u;
     // the next rebuild reorders when it is the first of a new group of reorder_every
     *w.reorder = (w.reorder_every <= 1 || n % (unsigned long long)w.reorder_every == 0ull) ? 1 : 0;
 }

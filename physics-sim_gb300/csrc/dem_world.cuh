@@ -135,6 +135,7 @@ struct StepRun {
     float *rec_out;
     uint32_t skew;           // the barrier counters' start, 0; else no barrier is ever complete (tests)
     struct RunReport *report;
+    uint32_t crowd;          // 1: the rebuild under way met more than CROWDED_ROW particles in a row of cells
     unsigned long long rebuilds, overflows;  // DevWorld::stats [4] and [5] when the report was last written
 };
 // What the host learns of the runs, in page-locked host memory.
@@ -142,7 +143,12 @@ struct RunReport {
     int32_t err;          // DevWorld::err as of the last wait for the stream (World::queue_check)
     int32_t failed;       // written by the device: a run before this one failed
     uint32_t overflows;   // by the device: particles whose list overflowed, a rebuild, of the latest rebuilds known
+    uint32_t crowd;       // by the device: StepRun::crowd of the last sorted rebuild
 };
+// Particles in a search's row of cells from which on a world is not rebuilt by
+// cell chains (World::crowded): a chain costs a trip to L2 a particle, ~0.5 us,
+// the sorted rebuild and the way to it ~150.
+constexpr int CROWDED_ROW = 256;
 // before every launch of the kernel
 __device__ __forceinline__ void clear_run_barrier(StepRun &R) {
     R.arrive[0] = R.arrive[1] = R.arrive[2] = R.skew;

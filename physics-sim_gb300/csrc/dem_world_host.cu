@@ -2015,9 +2015,15 @@ bool World::device_full() const {
 // rebuilds walk chains (microseconds a step by launches and by runs, disks
 // overlapping 5 to 10 deep: 3,000 462 / 534, 30,000 1,042 / 1,173, 100,000 692 /
 // 963, 250,000 2,101 / 3,975; packs of sizes 1 to 5 with 0.5 % of the lists
-// full 187 / 66 at 30,000 and 233 / 207 at 250,000).
+// full 187 / 66 at 30,000 and 233 / 207 at 250,000).  So does a world with a
+// crowded row of cells, as where particles thrown out of the search grid pile
+// up in its corner cell and move on at every step (400 of them 155 / 218, 3,600
+// 722 / 1,275, 50,176 9,214 / 23,567); a cell that fills during runs is seen
+// at the next rebuild that reorders, one in 32.
 bool World::crowded() const {
-    const long long over = report ? *(volatile uint32_t *)&report->overflows : 0;
+    if (!report) return false;
+    if (*(volatile uint32_t *)&report->crowd) return true;
+    const long long over = *(volatile uint32_t *)&report->overflows;
     if (over == 0) return false;
     long long n = 0;
     for (const auto &h : sh)

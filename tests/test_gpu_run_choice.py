@@ -157,3 +157,25 @@ def test_crowded_worlds_take_launches(n):
     assert calls[0] == 1, "nothing is known before the first rebuild"
     assert calls[2:6] == [0, 0, 0, 0], "most lists are full"
     assert calls[-1] == 1, "the disks have flown apart"
+
+
+def test_a_crowded_cell_takes_launches():
+    """Particles thrown out of the search grid share its corner cell; none is
+    near another, so no list is full."""
+    from test_gpu_parity import _append_particles
+
+    sc, p, _ = dem_scenes.dense_bed(2000, seed=5)
+    p = dict(p, round_bounds=1, bound_radius=1.0e6)
+    gx, gy = np.meshgrid(np.arange(40), np.arange(40))
+    x0 = sc["pos"].reshape(-1, 2).max(axis=0) + 10.0
+    at = np.stack([x0[0] + 4.0 * gx.ravel(), x0[1] + 4.0 * gy.ravel()], axis=1)
+    sc = _append_particles(sc, at, np.full(1600, 1.0), np.full((1600, 2), 1.0e7))
+    ref = copy_scene(sc)
+    with dem.Context(copy_scene(sc), p) as ctx:
+        for k, runs in enumerate((1, 0, 0)):  # the first rebuilds tell
+            before = ctx.run_calls()
+            ctx.step(40)
+            oracle.step(ref, p, 40)
+            assert_same_state(ctx.download(), ref, "call %d: " % k)
+            assert ctx.run_calls() - before == runs
+        assert ctx.stats()["list_overflows"] == 0
