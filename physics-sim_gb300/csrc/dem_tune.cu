@@ -16,7 +16,6 @@
 
 #include <algorithm>
 #include <chrono>
-#include <climits>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -44,12 +43,12 @@ struct Knobs {
 
 // ms per step of the sample with the given knobs: warm run (graph capture,
 // first rebuild), then `steps` timed steps with events on the world's stream.
-// launches: by launches whatever the sample's size; how: the way it stepped.
+// total: the batch's particles, which decide the way it steps; how: that way.
 struct How {
     bool runs = false, split = false;
 };
 int trial(const std::vector<const dem_scene *> &sc, const std::vector<dem_params> &ps,
-          const std::vector<dem_ext> &base, const Knobs &k, int steps, bool launches, double *ms_per_step,
+          const std::vector<dem_ext> &base, const Knobs &k, int steps, long long total, double *ms_per_step,
           How *how = nullptr) {
     std::vector<dem_ext> es = base;
     for (auto &e : es) {
@@ -72,7 +71,7 @@ int trial(const std::vector<const dem_scene *> &sc, const std::vector<dem_params
         cudaGetDevice(&w.device);
         rc = w.build(sc, ps, es);
         cudaEvent_t e0 = nullptr, e1 = nullptr;
-        if (rc == DEM_OK && launches) rc = w.set_runs(1);
+        if (rc == DEM_OK && !w.runs_fit(total)) rc = w.set_runs(1);
         if (rc == DEM_OK) rc = w.step(steps);
         if (how) *how = How{w.runs_resident(), w.d.split != 0};
         if (rc == DEM_OK && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess))
@@ -148,15 +147,14 @@ int dem_batch_autotune(const dem_scene *const *scenes, const dem_params *params,
     Knobs best;
     double best_ms = 0.0;
     int trials = 0;
-    const bool launches = total > INT_MAX || demgb::steps_block((int)total) == 0;
     How how;
-    int rc = trial(sc, ps, es, best, trial_steps, launches, &best_ms, &how);
+    int rc = trial(sc, ps, es, best, trial_steps, total, &best_ms, &how);
     if (rc) return rc;
     ++trials;
     const double default_ms = best_ms;
     auto try_knobs = [&](const Knobs &k) -> int {
         double ms = 0.0;
-        int r = trial(sc, ps, es, k, trial_steps, launches, &ms);
+        int r = trial(sc, ps, es, k, trial_steps, total, &ms);
         if (r) return r;
         ++trials;
         if (ms < best_ms) {

@@ -1664,14 +1664,15 @@ void World::enqueue_rebuild(cudaStream_t st, const int32_t *gate, bool every_ste
 // sparser worlds read the cell table directly (measured: the 4 M-particle
 // impact bed, 5.3 particles a cell, 0.59 -> 0.38 ms per list build staged;
 // the 512-scene mix, 0.74 a cell, 0.21 -> 0.44 ms)
-bool World::dense_cells() const {
+// (halves: that many halves a cell)
+bool World::dense_cells(int halves) const {
     long long cells = 0, n = 0;
     for (const auto &h : sh) {
         if (!h.active) continue;
         cells += (long long)h.par.g_w * h.par.g_h;
         n += h.n;
     }
-    return cells > 0 && 2 * n >= 3 * cells;
+    return cells > 0 && 2 * n >= halves * cells;
 }
 
 void World::rec_event(int kind, cudaStream_t st) {
@@ -1885,8 +1886,21 @@ int World::capture_run(cudaGraphExec_t *out) {
 // a step: 128 bonded particles 19.4 -> 4.2, 4,096 falling 13.8 -> 2.7, 16,384
 // bonded 18.2 -> 5.7, a 30,011-particle bed with F64 distances 35.9 -> 9.8, a
 // 262,144-particle bed 44.3 -> 31.4); k_big_narrow is a launch of its own.
+// Two particles a thread pay only where they have few neighbours: beyond one,
+// worlds of 2.5 particles a search cell or more (beds have 1.6, the mix 0.7,
+// packs and bonded packings 4) step by launches, whose kernels spill less and
+// hold more warps (launches / runs: 200,000 particles of a pack 46 / 71,
+// bonded by model 3 42 / 49, by model 2 41 / 58, 300,000 58 / 76, 51 / 53 and
+// 49 / 62; a bed of 200,000 35 / 32, of 300,000 43 / 33; up to 155,648 runs are
+// ahead everywhere, 150,000 of a pack 45 / 37, bonded 37 / 30).
+bool World::runs_fit(long long n) const {
+    const int threads = n == d.N ? run_block : n <= INT_MAX ? steps_block((int)n) : 0;
+    return threads > 0 &&
+           !(threads == SWEEP_THREADS && n > (long long)SWEEP_THREADS * device_sms() && dense_cells(5));
+}
+
 bool World::runs_resident() const {
-    return use_graphs && !timing && !has_bigs && run_block > 0 && !runs_refused && !runs_off;
+    return use_graphs && !timing && !has_bigs && !runs_refused && !runs_off && runs_fit(d.N);
 }
 
 // Whether the graph of a run is there or could be captured.  Where the device

@@ -138,6 +138,7 @@ class World {
     int fail_waits();  // debug
     static long long queued_on(int device);  // particles of the worlds with steps queued (DEVICES at most)
     bool runs_resident() const;    // step calls may be runs
+    bool runs_fit(long long n) const;  // n particles of this world's density
     long long run_calls = 0;       // step calls (and chunks of a record) taken as runs
     int set_runs(int mode);        // debug: 0 the library's choice, 1 launches, 2 every run refused
 
@@ -188,7 +189,7 @@ class World {
     int runs_intact();
     bool was_resident = false;
     void drop_graph();
-    bool dense_cells() const;
+    bool dense_cells(int halves = 3) const;
     DevWorld spare{};
     std::vector<void *> owned;
     // device copy of one scene in the reference layouts (uploads, downloads)

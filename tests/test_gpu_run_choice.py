@@ -179,3 +179,20 @@ def test_a_crowded_cell_takes_launches():
             assert_same_state(ctx.download(), ref, "call %d: " % k)
             assert ctx.run_calls() - before == runs
         assert ctx.stats()["list_overflows"] == 0
+
+
+def test_dense_worlds_of_two_particles_a_thread_take_launches():
+    from test_gpu_match_word import packed
+
+    for cols, runs in ((380, 1), (420, 0)):  # 144,400 and 176,400 particles
+        sc, p, ext = packed(2, cols, cols, 1.0)
+        ref = copy_scene(sc)
+        with dem.Context(copy_scene(sc), p, **ext) as ctx:
+            ctx.step(12)
+            oracle.step(ref, p, 12, **{k: ext[k] for k in ("bond_lambda", "bond_sn", "bond_ss") if k in ext})
+            assert_same_state(ctx.download(), ref)
+            assert ctx.run_calls() == runs
+    sc, p, ext = shaken_bed(176400, 2)
+    with dem.Context(sc, p, **ext) as ctx:
+        ctx.step(12)
+        assert ctx.run_calls() == 1
