@@ -465,6 +465,8 @@ def run_ours(args):
                 "algorithmic_bytes_per_launch": alg_bytes,
                 "slots_unbonded": s_u, "slots_bonded": s_b,
                 "lom_us": lom_ms / max(lom_n, 1) * 1e3, "broad_phase_us": bp_ms / max(bp_n, 1) * 1e3}
+    if ctx.run_calls() > 0:  # kernel timing steps by launches
+        roofline["note"] = "the launched kernel; the timed region stepped in runs (k_steps or k_sweep)"
 
     # end to end through the public API: restore from host arrays, one frame, update_state
     import dem as _dem

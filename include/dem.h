@@ -90,9 +90,10 @@ typedef struct dem_ext {
     const float *bond_shear_strength;
     int32_t diagnostics;              /* 1: maintain data[7n] every step as the reference does */
     int32_t reorder_interval;         /* steps per captured CUDA graph; 0 = library default (35).  Worlds
-                                         of up to 311,296 particles, none of them large, take a step
-                                         call in one kernel: reorder_interval, block_size,
-                                         split_narrow and unfused_lom have no effect there */
+                                         of up to 2,048 particles an SM (311,296), none of them large,
+                                         take a call of several steps in one kernel where the library
+                                         finds that faster: reorder_interval, block_size, split_narrow
+                                         and unfused_lom have no effect there */
     int32_t block_size;               /* threads per block for particle kernels; 0 = default */
     float search_cell_factor;         /* search-grid cell / (2 r_max + skin), in [0.5, inf); 0 = default
                                          1.0.  Below 1 the cell searches span 5 x 5 cells instead of
@@ -180,7 +181,9 @@ typedef struct dem_stats {
                                    kernel's wait for its own blocks ran out of time (the calls that
                                    wait or read state, and every step, then return DEM_E_TIMEOUT) */
     int32_t reserved;
-    int64_t kernel_launches;    /* kernels this library launched on the context's stream */
+    int64_t kernel_launches;    /* kernels the calls put on the context's stream, alone or in graphs;
+                                   not counted: what a graph's conditional bodies launch (rebuilds, and
+                                   a step kernel that goes on after one) */
     int64_t list_overflows;     /* particles whose candidates exceeded the list (searched the cells) */
 } dem_stats;
 

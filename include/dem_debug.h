@@ -34,7 +34,9 @@ int dem_debug_search_grid(dem_ctx *ctx, float *x0, float *y0, float *inv, int32_
  * (milliseconds) and launch count of one kernel kind since timing was
  * enabled: "interact", "lom", "end_step", and the rebuild's three phases
  * "broad_phase" (keys, cell table, sort, grouping), "reorder" and
- * "candidate_lists" (each launched, gated, at every step). */
+ * "candidate_lists" (each launched, gated, at every step).  A world whose step
+ * calls are one kernel otherwise (see dem_debug_runs) is timed as it would
+ * step by launches. */
 int dem_debug_kernel_timing(dem_ctx *ctx, int32_t enable);
 int dem_debug_kernel_time(dem_ctx *ctx, const char *kernel, double *total_ms, int64_t *launches);
 /* The same kernel timing for a batch. */

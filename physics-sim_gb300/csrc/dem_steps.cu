@@ -33,7 +33,8 @@ namespace {
 // 131,000-particle bed goes from 29.3 to 18.9 us and of 129,756 particles of
 // the mix from 22.0 to 14.0, with two of a 262,144-particle bed from 38.6 to
 // 31.5 (214,475 of the mix 23.8 -> 23.6); with three it gains nothing (400,000:
-// 46.0 -> 45.5) and beyond the launches' better balance wins.
+// 46.0 -> 45.5) and beyond the launches' better balance wins.  Worlds of many
+// neighbours a particle stop at one (World::runs_fit).
 constexpr int SWEEPS = 2;
 
 // Blocks of the cluster that holds a world of n particles, of tb threads each;

@@ -288,7 +288,8 @@ int launch_interact(const DevWorld &w, int block, cudaStream_t st, bool bigs, bo
                     bool in_graph, cudaGraphConditionalHandle cond, int form, const ScenePar *pv, int ps);
 
 // Runs of steps in one kernel (dem_steps.cu), for worlds of at most one
-// particle a thread, 512 threads an SM, without large particles.
+// particle a thread with 512 threads an SM, or two with 1,024, without large
+// particles.
 // steps_block: the block size for n particles, 0 when the device or the size
 // does not allow it.  launch_run_begin: the next run takes `todo` steps.
 // launch_steps: captured in a graph's while node; the kernel sets `rebuild`

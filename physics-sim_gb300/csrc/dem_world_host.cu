@@ -1881,11 +1881,13 @@ int World::capture_run(cudaGraphExec_t *out) {
     return DEM_OK;
 }
 
-// Whether a step call is one run of k_steps or k_sweep.  Every world whose
-// particles fit two a thread takes it (a launch a step -> a run, microseconds
-// a step: 128 bonded particles 19.4 -> 4.2, 4,096 falling 13.8 -> 2.7, 16,384
-// bonded 18.2 -> 5.7, a 30,011-particle bed with F64 distances 35.9 -> 9.8, a
-// 262,144-particle bed 44.3 -> 31.4); k_big_narrow is a launch of its own.
+// Whether a step call may be one run of k_steps or k_sweep: worlds whose
+// particles fit two a thread (a launch a step -> a run, microseconds a step of
+// a call of 105 and the wait for it: 128 bonded particles 17.1 -> 3.8, 4,096
+// falling 13.4 -> 2.6, 16,384 bonded 17.9 -> 5.6, a 30,011-particle bed with F64
+// distances 34.2 -> 9.6, a 262,144-particle bed 41.7 -> 33.1); k_big_narrow is
+// a launch of its own.
+//
 // Two particles a thread pay only where they have few neighbours: beyond one,
 // worlds of 2.5 particles a search cell or more (beds have 1.6, the mix 0.7,
 // packs and bonded packings 4) step by launches, whose kernels spill less and
