@@ -45,7 +45,8 @@ constexpr int SWEEPS = 2;
 // 8.0 -> 6.5.  One block alone loses (128 bonded 4.2 -> 4.75), and beyond 256
 // threads a block the warps would share their schedulers.
 int cluster_blocks(int n, int &tb) {
-    if (n <= TB_SMALL || n > 16 * TB_MID) return 0;
+    static_assert(16 * TB_MID == CLUSTER_MOST, "a cluster of 16 blocks");
+    if (n <= TB_SMALL || n > CLUSTER_MOST) return 0;
     tb = n <= 16 * TB_SMALL ? TB_SMALL : TB_MID;
     int blocks = 1;
     while (blocks * tb < n) blocks *= 2;

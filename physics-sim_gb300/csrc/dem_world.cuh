@@ -303,6 +303,7 @@ struct RunRecord {
 int device_sms();  // SMs of the current device
 constexpr int SWEEP_THREADS = 1024;  // block size of the worlds whose particles exceed the threads; they record no data
 constexpr int NARROW_BLOCK = 128;    // blocks of more threads leave no room for another world's on their SM
+constexpr int CLUSTER_MOST = 4096;   // particles of a world in one block or cluster
 int steps_block(int n);
 void launch_run_begin(const DevWorld &w, int todo, const RunRecord &rec, cudaStream_t st);
 cudaError_t launch_steps(const DevWorld &w, int block, cudaStream_t st, cudaGraphConditionalHandle more,

@@ -77,22 +77,22 @@ void RangeAlloc::release(long long off, long long n) {
 // only ever waits for a world's stream by itself leaves the world counted;
 // worlds of plain launches, which such hosts capture, are not.
 constexpr int DEVICES = 64;
-static std::atomic<long long> queued_particles[DEVICES];
+static std::atomic<long long> queued_particles[DEVICES], grid_particles[DEVICES];
 
-long long World::queued_on(int device) {
-    return device >= 0 && device < DEVICES ? queued_particles[device].load(std::memory_order_relaxed) : 0;
-}
-
-void World::count_queued() {
-    if (queued || !use_graphs || device < 0 || device >= DEVICES) return;
-    queued = d.N;
-    queued_particles[device].fetch_add(queued, std::memory_order_relaxed);
+void World::count_queued(bool run) {
+    if (!use_graphs || device < 0 || device >= DEVICES) return;
+    const auto count = [](std::atomic<long long> &all, long long &mine, long long n) {
+        if (n != mine) all.fetch_add(n - mine, std::memory_order_relaxed);
+        mine = n;
+    };
+    count(queued_particles[device], queued, d.N);
+    count(grid_particles[device], in_grid, run && d.N > CLUSTER_MOST ? d.N : 0);
 }
 
 void World::settled() {
-    if (!queued) return;
-    queued_particles[device].fetch_sub(queued, std::memory_order_relaxed);
-    queued = 0;
+    if (queued) queued_particles[device].fetch_sub(queued, std::memory_order_relaxed);
+    if (in_grid) grid_particles[device].fetch_sub(in_grid, std::memory_order_relaxed);
+    queued = in_grid = 0;
 }
 
 cudaError_t World::wait() {
@@ -1927,7 +1927,7 @@ bool World::run_steps(int n_steps, const RunRecord &rec) {
         runs_refused = true;
         return false;
     }
-    count_queued();
+    count_queued(true);
     ++run_calls;
     unchecked = true;
     launches += 2;
@@ -2020,10 +2020,21 @@ void World::update_split() {
 // ones, gain from runs (2 x 30,011 26 / 18, 8 x 16,384 62 / 35).  So such a
 // world takes launches while the queued worlds hold more than 512 particles an
 // SM with it, and for HOLD calls after, since the way back costs a rebuild.
+// Smaller grids share the SMs with each other, but they hold them at their
+// barriers against a world too large for runs (2,048 an SM), which then waits:
+// beside 1,000,000 particles they are runs while all of them hold half of the
+// SMs' blocks of 128 or less (the large world's and theirs: 4 x 16,384 by
+// launches 95 and 95, as runs 980 and 22; one of 5,000 97 and 11 as a run, 98
+// and 65 by launches).  Clusters of up to 16 SMs stay runs.
 constexpr int SINGLES = 32, HOLD = 16;
 bool World::device_full() const {
-    const long long others = queued_on(device) - queued;
-    return run_block > NARROW_BLOCK && others > 0 && others + d.N > 512LL * device_sms();
+    if (d.N <= CLUSTER_MOST || device < 0 || device >= DEVICES) return false;
+    const long long others = queued_particles[device].load(std::memory_order_relaxed) - queued;
+    if (others <= 0) return false;
+    const int sms = device_sms();
+    if (run_block > NARROW_BLOCK) return others + d.N > 512LL * sms;
+    const long long grids = grid_particles[device].load(std::memory_order_relaxed) - in_grid + d.N;
+    return others + d.N > 2048LL * sms && grids > 64LL * sms;
 }
 
 // Where most lists overflow their particles go over whole cells at every step:
@@ -2098,7 +2109,7 @@ int World::step(int n_steps) {
         rc = refresh_graphs(false);
         if (rc) return rc;
     }
-    count_queued();
+    count_queued(false);
     int k = 0;
     if (use_graphs && !timing && n_steps > 0) {
         while (n_steps - k >= graph_steps) {

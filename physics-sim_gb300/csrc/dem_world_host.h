@@ -136,7 +136,6 @@ class World {
     int kernel_time(int kind, double *ms, long long *n);
     void set_timing(bool on);
     int fail_waits();  // debug
-    static long long queued_on(int device);  // particles of the worlds with steps queued (DEVICES at most)
     bool runs_resident() const;    // step calls may be runs
     bool runs_fit(long long n) const;  // n particles of this world's density
     long long run_calls = 0;       // step calls (and chunks of a record) taken as runs
@@ -177,9 +176,10 @@ class World {
     bool crowded() const;
     int hold = 0;                  // step calls that stay launches
     // the world's particles while it has steps queued that no call has waited
-    // for, counted on its device
-    long long queued = 0;
-    void count_queued();
+    // for (in_grid: the last of them as a run over several blocks), counted on
+    // its device
+    long long queued = 0, in_grid = 0;
+    void count_queued(bool run);
     cudaError_t wait();            // for the stream
     void settled();
     cudaError_t queue_check();

@@ -107,6 +107,29 @@ def test_wide_runs_leave_the_device_to_others():
             assert_same_state(ctx.download(), ref)
 
 
+def test_grids_leave_a_large_world_its_sms():
+    """Beside a world too large for runs the small grids hold half of the SMs at
+    most; a cluster stays a run."""
+    sc, p, ext = shaken_bed(311297, 3)
+    worlds = [shaken_bed(n, n % 50) for n in (5000, 4800, 16000, 4000)]
+    refs = [copy_scene(w[0]) for w in worlds]
+    with dem.Context(sc, p, **ext) as big:
+        cs = [dem.Context(copy_scene(w[0]), w[1]) for w in worlds]
+        big.step(30)
+        for c in cs:
+            c.step(8)
+        # 5,000 alone is 40 blocks; with it 4,800 and 16,000 are too many
+        assert [c.run_calls() for c in cs] == [1, 0, 0, 1]
+        big.synchronize()
+        cs[0].synchronize()
+        for c in cs[:2]:
+            c.step(8)
+        for (_, q, _), ref, c, steps in zip(worlds, refs, cs, (16, 16, 8, 8)):
+            oracle.step(ref, q, steps)
+            assert_same_state(c.download(), ref)
+            c.close()
+
+
 def test_large_worlds_on_threads_of_their_own():
     import threading
 
