@@ -73,7 +73,7 @@ int steps_block(int n) {
 }
 
 cudaError_t launch_steps(const DevWorld &w, int block, cudaStream_t st, cudaGraphConditionalHandle more,
-                         cudaGraphConditionalHandle rebuild, int form, const ScenePar *pv, int ps) {
+                         cudaGraphConditionalHandle rebuild, int form, const ScenePar *pv, int ps, bool *waits) {
     const auto kernel = [&](int threads, bool cluster) {
         return form == 0 ? steps_kernel<0>(threads, cluster, ps)
                : form == 3 ? steps_kernel<3>(threads, cluster, ps)
@@ -86,6 +86,7 @@ cudaError_t launch_steps(const DevWorld &w, int block, cudaStream_t st, cudaGrap
     c.stream = st;
     c.attrs = &a;
     int tb = 0;
+    *waits = false;
     const int blocks = cluster_blocks(w.N, tb);
     if (blocks > 0) {
         // records in shared memory; a block an SM (two would share its schedulers)
@@ -126,6 +127,7 @@ cudaError_t launch_steps(const DevWorld &w, int block, cudaStream_t st, cudaGrap
     a.id = cudaLaunchAttributeCooperative;
     a.val.cooperative = 1;
     c.numAttrs = grid > 1 ? 1 : 0;
+    *waits = grid > 1;
     return cudaLaunchKernelEx(&c, fn, w, more, rebuild, par);
 }
 

@@ -306,8 +306,9 @@ constexpr int NARROW_BLOCK = 128;    // blocks of more threads leave no room for
 constexpr int CLUSTER_MOST = 4096;   // particles of a world in one block or cluster
 int steps_block(int n);
 void launch_run_begin(const DevWorld &w, int todo, const RunRecord &rec, cudaStream_t st);
+// waits: whether blocks wait for one another in software, which may give up
 cudaError_t launch_steps(const DevWorld &w, int block, cudaStream_t st, cudaGraphConditionalHandle more,
-                         cudaGraphConditionalHandle rebuild, int form, const ScenePar *pv, int ps);
+                         cudaGraphConditionalHandle rebuild, int form, const ScenePar *pv, int ps, bool *waits);
 
 // The fields of a scene's parameters that the Simulation kernels read from
 // the launch under PS_SHARED (the settings and model constants), the others

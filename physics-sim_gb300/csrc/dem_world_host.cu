@@ -103,7 +103,7 @@ cudaError_t World::wait() {
 
 // the device's error word for runs_intact() after the next wait; ahead of a
 // call's own copies, which then hide most of it (3 us; behind them 7).  Only
-// runs wait between blocks.
+// runs over several blocks wait for one another, and a cluster's in hardware.
 cudaError_t World::queue_check() {
     if (!unchecked) return cudaSuccess;
     unchecked = false;
@@ -1853,7 +1853,7 @@ int World::capture_run(cudaGraphExec_t *out) {
     if (e == cudaSuccess) {
         cudaGraph_t done = nullptr;
         e = runs_fault ? cudaErrorCooperativeLaunchTooLarge
-                       : launch_steps(d, run_block, side, more, due, kernel_form, &par_pv, par_ps);
+                       : launch_steps(d, run_block, side, more, due, kernel_form, &par_pv, par_ps, &run_waits);
         const cudaGraphNode_t *deps = nullptr;
         size_t ndeps = 0;
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -1929,7 +1929,7 @@ bool World::run_steps(int n_steps, const RunRecord &rec) {
     }
     count_queued(true);
     ++run_calls;
-    unchecked = true;
+    unchecked |= run_waits;
     launches += 2;
     host_step += n_steps;
     return true;

@@ -183,7 +183,8 @@ class World {
     cudaError_t wait();            // for the stream
     void settled();
     cudaError_t queue_check();
-    bool unchecked = false;        // a run since the last queue_check
+    bool unchecked = false;        // a run whose waits may have given up since the last queue_check
+    bool run_waits = false;        // whether a run has such waits (launch_steps)
     int singles = 0;               // step calls of one step in a row, while they are runs
     RunReport *report = nullptr;   // page-locked (StepRun::report)
     int runs_intact();
